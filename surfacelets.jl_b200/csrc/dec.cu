@@ -17,7 +17,7 @@
 #include <cmath>
 #include <cstring>
 
-#include "passes.cuh"
+#include "mixpass.cuh"
 #include "plan.h"
 #include "regpass.cuh"
 #include "slab_core.cuh"
@@ -586,59 +586,8 @@ struct BlockMap {
     }
 };
 
-// C2R output of two block lines into the subbands (element stride es).
-struct StoreRPairBlocks {
-    float* dst;
-    BlockMap bm;
-    int nlines;
-    int es;
-    __device__ __forceinline__ void operator()(const float2* tile, int npad, int n, int l0, int T, int) const {
-        const int total = T * n;
-        const bool ifast = bm.K == 0;
-        for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-            int t, i;
-            if (ifast) {
-                i = idx % n;
-                t = idx / n;
-            } else {
-                t = idx % T;
-                i = idx / T;
-            }
-            int la = 2 * (l0 + t);
-            float2 v = tile[t * npad + i];
-            if (la < nlines) dst[bm.addr(la, i) * es] = v.x;
-            if (la + 1 < nlines) dst[bm.addr(la + 1, i) * es] = v.y;
-        }
-    }
-};
-
-// Two subband lines along K packed as one complex line (R2C input).
-struct LoadRPairBlocks {
-    const float* src;
-    BlockMap bm;
-    int nlines;
-    int es;
-    __device__ __forceinline__ void operator()(float2* tile, int npad, int n, int l0, int T, int) const {
-        const int total = T * n;
-        const bool ifast = bm.K == 0;
-        for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-            int t, i;
-            if (ifast) {
-                i = idx % n;
-                t = idx / n;
-            } else {
-                t = idx % T;
-                i = idx / T;
-            }
-            int la = 2 * (l0 + t);
-            float a = la < nlines ? src[bm.addr(la, i) * es] : 0.f;
-            float b = la + 1 < nlines ? src[bm.addr(la + 1, i) * es] : 0.f;
-            tile[t * npad + i] = make_float2(a, b);
-        }
-    }
-};
-
-// Register-pass versions of the two block ops (see regpass.cuh).
+// Two block lines out to (C2R) and in from (R2C) the subbands, element stride
+// es.
 struct RStoreRPairBlocks {
     static constexpr bool kStaged = false;
     float* dst;
@@ -820,22 +769,12 @@ unsigned grid_for(long long total) {
 void fft_real_full(DecPlan& D, const float* x, int es, const int d[3], float2* X, cudaStream_t st) {
     Lines gin = axis_lines(d, 0);
     FFTLen* f0 = get_fft(D.ffts, d[0]);
-    int pairs = (gin.nlines + 1) / 2;
-    if (!launch_reg<false>(d[0], RLoadRPair{x, ZMap{}, gin, es}, RStoreFullPair{X, ZMap{}, gin, d[0]}, f0->sh.tw,
-                           pairs, 1, false, st, "dec_fft_r2c")) {
-        LoadRPair ld{x, ZMap{}, gin, es};
-        StoreFullPair sto{X, ZMap{}, gin};
-        launch_pass(ld, sto, f0->sh, pairs, 1, false, st, "dec_fft_r2c");
-    }
+    launch_line<false>(*f0, RLoadRPair{x, ZMap{}, gin, es}, RStoreFullPair{X, ZMap{}, gin, d[0]}, (gin.nlines + 1) / 2,
+                       1, false, st, "dec_fft_r2c");
     for (int a = 1; a < 3; ++a) {
         Lines g = axis_lines(d, a);
-        FFTLen* f = get_fft(D.ffts, d[a]);
-        if (launch_reg<false>(d[a], RLoadC{X, ZMap{}, g}, RStoreC{X, ZMap{}, g}, f->sh.tw, g.nlines, 1, true, st,
-                              "dec_fft_c2c"))
-            continue;
-        LoadC l2{X, ZMap{}, g, 1.f};
-        StoreC s2{X, ZMap{}, g, 1.f};
-        launch_pass(l2, s2, f->sh, g.nlines, 1, false, st, "dec_fft_c2c");
+        launch_line<false>(*get_fft(D.ffts, d[a]), RLoadC{X, ZMap{}, g}, RStoreC{X, ZMap{}, g}, g.nlines, 1, true, st,
+                           "dec_fft_c2c");
     }
 }
 
@@ -843,22 +782,12 @@ void fft_real_full(DecPlan& D, const float* x, int es, const int d[3], float2* X
 void ifft_full_real(DecPlan& D, float2* X, const int d[3], float* out, int es, float scale, cudaStream_t st) {
     for (int a = 2; a >= 1; --a) {
         Lines g = axis_lines(d, a);
-        FFTLen* f = get_fft(D.ffts, d[a]);
-        if (launch_reg<true>(d[a], RLoadC{X, ZMap{}, g}, RStoreC{X, ZMap{}, g}, f->sh.tw, g.nlines, 1, true, st,
-                             "dec_fft_c2c"))
-            continue;
-        LoadC l2{X, ZMap{}, g, 1.f};
-        StoreC s2{X, ZMap{}, g, 1.f};
-        launch_pass(l2, s2, f->sh, g.nlines, 1, true, st, "dec_fft_c2c");
+        launch_line<true>(*get_fft(D.ffts, d[a]), RLoadC{X, ZMap{}, g}, RStoreC{X, ZMap{}, g}, g.nlines, 1, true, st,
+                          "dec_fft_c2c");
     }
     Lines g0 = axis_lines(d, 0);
-    FFTLen* f0 = get_fft(D.ffts, d[0]);
-    if (launch_reg<true>(d[0], RLoadC{X, ZMap{}, g0}, RStoreReal{out, ZMap{}, g0, es, scale}, f0->sh.tw, g0.nlines,
-                         1, false, st, "dec_fft_real"))
-        return;
-    LoadC l0{X, ZMap{}, g0, 1.f};
-    StoreReal s0{out, ZMap{}, g0, es, scale};
-    launch_pass(l0, s0, f0->sh, g0.nlines, 1, true, st, "dec_fft_real");
+    launch_line<true>(*get_fft(D.ffts, d[0]), RLoadC{X, ZMap{}, g0}, RStoreReal{out, ZMap{}, g0, es, scale}, g0.nlines,
+                      1, false, st, "dec_fft_real");
 }
 
 // Lines of the segmented FFTs along axis m of a half-K spectrum (dims hd):
@@ -884,18 +813,14 @@ Lines block_lines(const int hd[3], int m, int bl) {
 void block_fft(DecPlan& D, float2* S, const int hd[3], int m, int bl, bool inv, cudaStream_t st) {
     const Lines g = block_lines(hd, m, bl);
     FFTLen* f = get_fft(D.ffts, bl);
-    bool tf = g.si != 1;
-    bool done = inv ? launch_reg<true>(bl, RLoadC{S, ZMap{}, g}, RStoreC{S, ZMap{}, g}, f->sh.tw, g.nlines, 1, tf, st,
-                                       "dec_block_fft")
-                    : launch_reg<false>(bl, RLoadC{S, ZMap{}, g}, RStoreC{S, ZMap{}, g}, f->sh.tw, g.nlines, 1, tf,
-                                        st, "dec_block_fft");
-    if (done) return;
-    LoadC ld{S, ZMap{}, g, 1.f};
-    StoreC sto{S, ZMap{}, g, 1.f};
-    launch_pass(ld, sto, f->sh, g.nlines, 1, inv, st, "dec_block_fft");
+    const bool tf = g.si != 1;
+    if (inv)
+        launch_line<true>(*f, RLoadC{S, ZMap{}, g}, RStoreC{S, ZMap{}, g}, g.nlines, 1, tf, st, "dec_block_fft");
+    else
+        launch_line<false>(*f, RLoadC{S, ZMap{}, g}, RStoreC{S, ZMap{}, g}, g.nlines, 1, tf, st, "dec_block_fft");
 }
 
-// Block FFTs of several spectra in one register pass: item z (grid.y) has its
+// Block FFTs of several spectra in one pass: item z (grid.y) has its
 // own spectrum and line geometry (same length); lines past an item's count
 // read zeros and store nothing.
 constexpr int kMaxLineJobs = 6;
@@ -935,7 +860,7 @@ struct RStoreCJobs {
 };
 
 // Up to three line passes of one loader / store type as the jobs of one
-// register-pass launch (grid.y = job): each job keeps its own geometry, and
+// launch (grid.y = job): each job keeps its own geometry, and
 // lines past a job's own count are invalid for it.
 template <class L>
 struct LoadJobs {
@@ -963,8 +888,7 @@ struct StoreJobs {
 };
 
 // The block FFTs of every hourglass of level L along both transverse axes,
-// grouped into one launch per (block length, line layout); lengths without a
-// register pass run one segmented pass per spectrum and axis.
+// grouped into one launch per (block length, line layout).
 void block_fft_level(DecPlan& D, DecLevelDev& L, bool inv, const bool skip[3], cudaStream_t st) {
     struct Item {
         int K, m, bl;
@@ -979,7 +903,6 @@ void block_fft_level(DecPlan& D, DecLevelDev& L, bool inv, const bool skip[3], c
     for (int a = 0; a < ni; ++a) {
         if (items[a].done) continue;
         LineJobs jobs;
-        int member[kMaxLineJobs];   // the item of each job
         int nlines = 0;
         bool inGroup[3] = {false, false, false};
         for (int b = a; b < ni; ++b) {
@@ -992,7 +915,6 @@ void block_fft_level(DecPlan& D, DecLevelDev& L, bool inv, const bool skip[3], c
                 if (items[c].K == K && !items[c].done) earlier_pending = true;
             if (inGroup[K] || earlier_pending) continue;
             inGroup[K] = true;
-            member[jobs.n] = b;
             jobs.base[jobs.n] = L.S[K].as<float2>();
             jobs.g[jobs.n] = block_lines(L.hd[K], items[b].m, items[b].bl);
             nlines = std::max(nlines, jobs.g[jobs.n].nlines);
@@ -1001,17 +923,11 @@ void block_fft_level(DecPlan& D, DecLevelDev& L, bool inv, const bool skip[3], c
         }
         const int bl = items[a].bl;
         FFTLen* f = get_fft(D.ffts, bl);
-        const bool ok = inv ? launch_reg<true>(bl, RLoadCJobs{jobs}, RStoreCJobs{jobs}, f->sh.tw, nlines, jobs.n,
-                                               items[a].tf, st, "dec_block_fft")
-                            : launch_reg<false>(bl, RLoadCJobs{jobs}, RStoreCJobs{jobs}, f->sh.tw, nlines, jobs.n,
-                                                items[a].tf, st, "dec_block_fft");
-        if (!ok) {
-            // no register pass for this length: one generic segmented pass per spectrum and axis
-            for (int t = 0; t < jobs.n; ++t) {
-                const Item& it = items[member[t]];
-                block_fft(D, jobs.base[t], L.hd[it.K], it.m, bl, inv, st);
-            }
-        }
+        if (inv)
+            launch_line<true>(*f, RLoadCJobs{jobs}, RStoreCJobs{jobs}, nlines, jobs.n, items[a].tf, st, "dec_block_fft");
+        else
+            launch_line<false>(*f, RLoadCJobs{jobs}, RStoreCJobs{jobs}, nlines, jobs.n, items[a].tf, st,
+                               "dec_block_fft");
     }
 }
 
@@ -1246,14 +1162,7 @@ void scale_forward(DecPlan& D, int j, float* c, int es, cudaStream_t st) {
             ++nj;
         }
         FFTLen* f = get_fft(D.ffts, L.n[K]);
-        if (!launch_reg<true>(L.n[K], lj, sj, f->sh.tw, pairs, nj, K != 0, st, "dec_c2r_blocks")) {
-            for (int t = 0; t < nj; ++t) {
-                const RLoadHPair& l1 = lj.j[t];
-                LoadHPair ld{l1.src, ZMap{}, l1.g};
-                StoreRPairBlocks sto{c, sj.j[t].bm, l1.g.nlines, es};
-                launch_pass(ld, sto, f->sh, (l1.g.nlines + 1) / 2, 1, true, st, "dec_c2r_blocks");
-            }
-        }
+        launch_line<true>(*f, lj, sj, pairs, nj, K != 0, st, "dec_c2r_blocks");
     }
 }
 
@@ -1281,14 +1190,7 @@ void scale_inverse(DecPlan& D, int j, const float* c, int es, cudaStream_t st) {
             ++nj;
         }
         FFTLen* f = get_fft(D.ffts, L.n[K]);
-        if (!launch_reg<false>(L.n[K], lj, sj, f->sh.tw, pairs, nj, K != 0, st, "dec_r2c_blocks")) {
-            for (int t = 0; t < nj; ++t) {
-                const RStoreHalfPair& s1 = sj.j[t];
-                LoadRPairBlocks ld{c, lj.j[t].bm, s1.g.nlines, es};
-                StoreHalfPair sto{s1.dst, ZMap{}, s1.g};
-                launch_pass(ld, sto, f->sh, (s1.g.nlines + 1) / 2, 1, false, st, "dec_r2c_blocks");
-            }
-        }
+        launch_line<false>(*f, lj, sj, pairs, nj, K != 0, st, "dec_r2c_blocks");
     }
     // the block FFTs of the hourglasses whose plane pass does not run them, grouped by length and layout
     bool fuse[3];
@@ -1367,13 +1269,8 @@ void scale_forward_adjoint(DecPlan& D, int j, const float* c, int es, cudaStream
         FFTLen* f = get_fft(D.ffts, L.n[K]);
         BlockMap bm = block_map(L, K);
         int pairs = (gk.nlines + 1) / 2;
-        if (!launch_reg<false>(L.n[K], RLoadRPairBlocks{c, bm, gk.nlines, es},
-                               RStoreHalfPair{S, ZMap{}, gk, L.n[K], 2.f}, f->sh.tw, pairs, 1, K != 0, st,
-                               "dec_r2c_blocks")) {
-            LoadRPairBlocks ld{c, bm, gk.nlines, es};
-            StoreHalfPair sto{S, ZMap{}, gk, 2.f};
-            launch_pass(ld, sto, f->sh, pairs, 1, false, st, "dec_r2c_blocks");
-        }
+        launch_line<false>(*f, RLoadRPairBlocks{c, bm, gk.nlines, es}, RStoreHalfPair{S, ZMap{}, gk, L.n[K], 2.f}, pairs,
+                           1, K != 0, st, "dec_r2c_blocks");
         for (int m = 0; m < 3; ++m)
             if (m != K) block_fft(D, S, hd, m, L.bsize[K][m], false, st);
         for (int sg_i = (int)L.stages[K].size() - 1; sg_i >= 0; --sg_i) {
@@ -1426,12 +1323,8 @@ void scale_inverse_adjoint(DecPlan& D, int j, float* c, int es, cudaStream_t st)
         FFTLen* f = get_fft(D.ffts, L.n[K]);
         BlockMap bm = block_map(L, K);
         int pairs = (gk.nlines + 1) / 2;
-        if (!launch_reg<true>(L.n[K], RLoadHPair{S, ZMap{}, gk, L.n[K], 0.5f}, RStoreRPairBlocks{c, bm, gk.nlines, es},
-                              f->sh.tw, pairs, 1, K != 0, st, "dec_c2r_blocks")) {
-            LoadHPair ld{S, ZMap{}, gk, 0.5f};
-            StoreRPairBlocks sto{c, bm, gk.nlines, es};
-            launch_pass(ld, sto, f->sh, pairs, 1, true, st, "dec_c2r_blocks");
-        }
+        launch_line<true>(*f, RLoadHPair{S, ZMap{}, gk, L.n[K], 0.5f}, RStoreRPairBlocks{c, bm, gk.nlines, es}, pairs, 1,
+                          K != 0, st, "dec_c2r_blocks");
     }
 }
 

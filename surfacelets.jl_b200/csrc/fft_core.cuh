@@ -1,11 +1,5 @@
-// Shared-memory mixed-radix Stockham FFT core for sm_100a, and the line
-// geometry the pass kernels use to stage tiles of lines through it.
-//
-// A CTA stages T lines of length n in shared memory (row pitch npad = n + 1
-// so that 64-bit accesses of consecutive lines hit distinct banks), runs the
-// Stockham stages with radix 8, 5, 4, 3, 2 (and a direct DFT for any other
-// prime factor), and hands the tile back to a store op.  Twiddles come from a
-// float64-designed table of e^{-2 pi i t/n}, staged in shared memory.
+// Complex arithmetic on register pairs, the radix-2/3/4/5/8 butterflies, and
+// the line geometry that the pass kernels share.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -13,13 +7,18 @@
 
 namespace sfl {
 
-constexpr int kMaxStages = 24;
-
 struct FFTShape {
     int n = 1;
-    int nstages = 0;
-    int radix[kMaxStages] = {};
-    const float2* tw = nullptr;   // device: n entries, e^{-2 pi i t / n}
+    const float2* tw = nullptr;   // device: n entries, e^{-2 pi i t / n}, float64-designed
+};
+
+// Radices of the mixed-radix line pass (mixpass.cuh) of a length, in step
+// order: its large prime factors, then radices of at most 20.
+constexpr int kMixMaxSteps = 8;
+struct MixSchedule {
+    int n = 1;
+    int ns = 0;
+    int R[kMixMaxSteps] = {};
 };
 
 // Complex arithmetic on (re, im) register pairs.  Additions, subtractions and
@@ -157,90 +156,6 @@ struct Dft<8> {
     }
 };
 
-__device__ __forceinline__ float2 twiddle(const float2* tw, int idx, bool inv) {
-    float2 w = tw[idx];
-    return inv ? make_float2(w.x, -w.y) : w;
-}
-
-// One Stockham stage of radix R over T lines (in -> out).
-template <int R>
-__device__ __forceinline__ void stockham_stage(const float2* __restrict__ in, float2* __restrict__ out, int T,
-                                               int n, int npad, int Ns, const float2* tw, bool inv) {
-    const int nb = n / R;
-    const int total = T * nb;
-    const int tstep = n / (Ns * R);
-    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-        int t = idx / nb;
-        int j = idx - t * nb;
-        const float2* x = in + t * npad;
-        float2* y = out + t * npad;
-        int k = j % Ns;
-        float2 v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = x[j + r * nb];
-        if (Ns > 1) {
-            int step = k * tstep;
-#pragma unroll
-            for (int r = 1; r < R; ++r) v[r] = c_mul(v[r], twiddle(tw, r * step, inv));
-        }
-        Dft<R>::run(v, inv);
-        int base = (j / Ns) * Ns * R + k;
-#pragma unroll
-        for (int r = 0; r < R; ++r) y[base + r * Ns] = v[r];
-    }
-}
-
-// A stage of any radix R (used for prime factors without a dedicated
-// butterfly): each output is a direct sum over the R inputs.
-__device__ __forceinline__ void stockham_stage_generic(const float2* __restrict__ in, float2* __restrict__ out,
-                                                       int R, int T, int n, int npad, int Ns, const float2* tw,
-                                                       bool inv) {
-    const int nb = n / R;
-    const int total = T * nb * R;
-    const int tstep = n / (Ns * R);
-    const int rstep = n / R;
-    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-        int m = idx % R;
-        int q = idx / R;
-        int t = q / nb;
-        int j = q - t * nb;
-        const float2* x = in + t * npad;
-        float2* y = out + t * npad;
-        int k = j % Ns;
-        float2 acc = make_float2(0.f, 0.f);
-        for (int r = 0; r < R; ++r) {
-            float2 v = x[j + r * nb];
-            if (Ns > 1 && r > 0) v = c_mul(v, twiddle(tw, r * k * tstep, inv));
-            int e = (r * m) % R;
-            acc = c_add(acc, e ? c_mul(v, twiddle(tw, e * rstep, inv)) : v);
-        }
-        y[(j / Ns) * Ns * R + k + m * Ns] = acc;
-    }
-}
-
-// All stages; returns the buffer that holds the result (a or b).
-__device__ __forceinline__ float2* fft_tile(float2* a, float2* b, int T, const FFTShape& sh, int npad,
-                                            const float2* tw, bool inv) {
-    int Ns = 1;
-    for (int s = 0; s < sh.nstages; ++s) {
-        int R = sh.radix[s];
-        switch (R) {
-            case 2: stockham_stage<2>(a, b, T, sh.n, npad, Ns, tw, inv); break;
-            case 3: stockham_stage<3>(a, b, T, sh.n, npad, Ns, tw, inv); break;
-            case 4: stockham_stage<4>(a, b, T, sh.n, npad, Ns, tw, inv); break;
-            case 5: stockham_stage<5>(a, b, T, sh.n, npad, Ns, tw, inv); break;
-            case 8: stockham_stage<8>(a, b, T, sh.n, npad, Ns, tw, inv); break;
-            default: stockham_stage_generic(a, b, R, T, sh.n, npad, Ns, tw, inv); break;
-        }
-        __syncthreads();
-        float2* t = a;
-        a = b;
-        b = t;
-        Ns *= R;
-    }
-    return a;
-}
-
 // Lines of a strided array: line l -> (l0, l1, l2) with l0 fastest; element i
 // of line l sits at l0*s0 + l1*s1 + l2*s2 + i*si.
 struct Lines {
@@ -268,10 +183,5 @@ struct Lines {
         return (long long)l0 * s0 + (long long)l1 * s1 + (long long)l2 * s2;
     }
 };
-
-// Shared-memory layout of a pass: [twiddles n][tile a T*npad][tile b T*npad] (+ extra).
-__device__ __forceinline__ void load_twiddles(float2* tws, const FFTShape& sh) {
-    for (int i = threadIdx.x; i < sh.n; i += blockDim.x) tws[i] = sh.tw[i];
-}
 
 }  // namespace sfl

@@ -35,7 +35,6 @@
 #include <mutex>
 
 #include "ns_mask.cuh"
-#include "passes.cuh"
 #include "plan.h"
 #include "regpass.cuh"
 
@@ -97,47 +96,33 @@ void ns_analyze_subband_static(NSPlan& P, const void* x, void* band, int index, 
     {
         FFTLen* f = planned_fft(P, P.dims[0]);
         Lines gin = axis_lines(P.dims, 0), gout = axis_lines(hd, 0);
-        int pairs = (gin.nlines + 1) / 2;
-        if (!launch_reg<false>(f->sh.n, RLoadRPair{xin, ZMap{}, gin, 1}, RStoreHalfPair{X, ZMap{}, gout, f->sh.n},
-                               f->sh.tw, pairs, 1, false, st, "ns_static_r2c"))
-            launch_pass(LoadRPair{xin, ZMap{}, gin, 1}, StoreHalfPair{X, ZMap{}, gout}, f->sh, pairs, 1, false, st,
-                        "ns_static_r2c");
+        launch_line<false>(*f, RLoadRPair{xin, ZMap{}, gin, 1}, RStoreHalfPair{X, ZMap{}, gout, f->sh.n},
+                           (gin.nlines + 1) / 2, 1, false, st, "ns_static_r2c");
     }
     for (int a = 1; a < 3; ++a) {
         FFTLen* f = planned_fft(P, hd[a]);
         Lines g = axis_lines(hd, a);
-        if (!launch_reg<false>(f->sh.n, RLoadC{X, ZMap{}, g}, RStoreC{X, ZMap{}, g}, f->sh.tw, g.nlines, 1, true, st,
-                               "ns_static_c2c"))
-            launch_pass(LoadC{X, ZMap{}, g, 1.f}, StoreC{X, ZMap{}, g, 1.f}, f->sh, g.nlines, 1, false, st,
-                        "ns_static_c2c");
+        launch_line<false>(*f, RLoadC{X, ZMap{}, g}, RStoreC{X, ZMap{}, g}, g.nlines, 1, true, st, "ns_static_c2c");
     }
     // c = irfft3(X * M): masked inverse pass along axis 3, axis 2, then C2R
     {
         FFTLen* f = planned_fft(P, hd[2]);
         Lines g = axis_lines(hd, 2);
         const NSItem* it = P.items.as<NSItem>();
-        if (!launch_reg<true>(f->sh.n, RLoadNSMask{X, P.tb, it, item, 0}, RStoreC{W, ZMap{}, g}, f->sh.tw, g.nlines,
-                              1, true, st, "ns_static_mask"))
-            launch_pass(LoadNSMask{X, P.tb, it, item, 0}, StoreC{W, ZMap{}, g, 1.f}, f->sh, g.nlines, 1, true, st,
-                        "ns_static_mask");
+        launch_line<true>(*f, RLoadNSMask{X, P.tb, it, item, 0}, RStoreC{W, ZMap{}, g}, g.nlines, 1, true, st,
+                          "ns_static_mask");
     }
     {
         FFTLen* f = planned_fft(P, hd[1]);
         Lines g = axis_lines(hd, 1);
-        if (!launch_reg<true>(f->sh.n, RLoadC{W, ZMap{}, g}, RStoreC{W, ZMap{}, g}, f->sh.tw, g.nlines, 1, true, st,
-                              "ns_static_c2c"))
-            launch_pass(LoadC{W, ZMap{}, g, 1.f}, StoreC{W, ZMap{}, g, 1.f}, f->sh, g.nlines, 1, true, st,
-                        "ns_static_c2c");
+        launch_line<true>(*f, RLoadC{W, ZMap{}, g}, RStoreC{W, ZMap{}, g}, g.nlines, 1, true, st, "ns_static_c2c");
     }
     {
         FFTLen* f = planned_fft(P, P.dims[0]);
         Lines gin = axis_lines(hd, 0), gout = axis_lines(P.dims, 0);
-        int pairs = (gout.nlines + 1) / 2;
         float scale = 1.0f / (float)P.N;
-        if (!launch_reg<true>(f->sh.n, RLoadHPair{W, ZMap{}, gin, f->sh.n}, RStoreRPair{out, ZMap{}, gout, 1, scale},
-                              f->sh.tw, pairs, 1, false, st, "ns_static_c2r"))
-            launch_pass(LoadHPair{W, ZMap{}, gin}, StoreRPair{out, ZMap{}, gout, 1, scale}, f->sh, pairs, 1, true, st,
-                        "ns_static_c2r");
+        launch_line<true>(*f, RLoadHPair{W, ZMap{}, gin, f->sh.n}, RStoreRPair{out, ZMap{}, gout, 1, scale},
+                          (gout.nlines + 1) / 2, 1, false, st, "ns_static_c2r");
     }
 }
 

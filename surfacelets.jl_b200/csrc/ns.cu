@@ -25,81 +25,62 @@
 
 namespace sfl {
 
-constexpr int kAccMax = 16;   // accumulator registers per thread (tile elements / 256)
+constexpr int kAccMaxLine = 4096;   // longest axis 3 of the accumulating pass without a register FFT
 
-// Pass 3 of the synthesis: for every item of the group, load its lines along
-// axis 3 from work + z*H, FFT, multiply by its mask and accumulate, with Kahan
-// compensation, into registers; then one round trip of acc/comp.
-__global__ void __launch_bounds__(256) ns_accum_kernel(const float2* __restrict__ work, long long H, int G,
-                                                       NSMaskTables tb, const NSItem* __restrict__ items,
-                                                       int item0, int synth, float2* acc, float2* comp, int init,
-                                                       FFTShape sh, int T, int npad) {
+// Pass 3 of the synthesis, any length: every item of the group is transformed
+// along axis 3 by the mixed-radix pass, multiplied by its mask and added, with
+// Kahan compensation, to the tile's sums in shared memory; then one round trip
+// of acc / comp.
+struct MixAccum {
+    static constexpr bool kStaged = false;
+    NSMaskTables tb;
+    const NSItem* items;
+    int item0, synth, l0, pitch;
+    float2* sums;   // tile sums, then their compensations
+    int comp;       // offset of the compensations
+    struct Ctx {
+        NSMaskLine m;
+        float2* s;
+    };
+    __device__ __forceinline__ Ctx line(int z, int l, bool) const {
+        return Ctx{ns_mask_line(tb, items[item0 + z], l, synth != 0), sums + (l - l0) * pitch};
+    }
+    __device__ __forceinline__ void put(const Ctx& c, int k, float2 v) const {
+        kahan_add(c.s[k], c.s[k + comp], c_scale(v, ns_mask_at(c.m, k, (long long)tb.h1 * tb.n2)));
+    }
+};
+
+template <bool BIG>
+__global__ void __launch_bounds__(256, 2) ns_accum_mix_kernel(const float2* __restrict__ work, long long H, int G,
+                                                              NSMaskTables tb, const NSItem* __restrict__ items,
+                                                              int item0, int synth, float2* acc, float2* comp, int init,
+                                                              MixArgs a) {
     extern __shared__ float2 smem[];
-    float2* tw = smem;
-    float2* a = smem + sh.n + (sh.n & 1);
-    float2* b = a + T * npad;
-    load_twiddles(tw, sh);
-    const int n = sh.n;
-    const int nlines = tb.h1 * tb.n2;
+    const int tsz = a.pitch << a.lg, LP = 1 << a.lg, l0 = blockIdx.x << a.lg, n = a.sc.n;
     const long long si = (long long)tb.h1 * tb.n2;
-    const int l0 = blockIdx.x * T;
-    const int total = T * n;
-    float2 s[kAccMax], c[kAccMax];
-#pragma unroll
-    for (int e = 0; e < kAccMax; ++e) {
-        s[e] = make_float2(0.f, 0.f);
-        c[e] = make_float2(0.f, 0.f);
+    float2* sums = smem;
+    float2* tile = smem + 2 * tsz;
+    for (int it = threadIdx.x; it < n << a.lg; it += blockDim.x) {
+        const int t = it & (LP - 1), i = it >> a.lg;
+        const bool have = !init && l0 + t < a.nlines;
+        sums[t * a.pitch + i] = have ? acc[l0 + t + i * si] : make_float2(0.f, 0.f);
+        sums[tsz + t * a.pitch + i] = have ? comp[l0 + t + i * si] : make_float2(0.f, 0.f);
     }
-    if (!init) {
-#pragma unroll
-        for (int e = 0; e < kAccMax; ++e) {
-            int idx = threadIdx.x + e * blockDim.x;
-            if (idx < total) {
-                int t = idx % T, i = idx / T, l = l0 + t;
-                if (l < nlines) {
-                    s[e] = acc[l + (long long)i * si];
-                    c[e] = comp[l + (long long)i * si];
-                }
-            }
-        }
-    }
+    RLoadC ld{work, ZMap{}, Lines{}};
+    ld.zm.zstride = H;
+    ld.g.si = si;
+    ld.g.B0 = a.nlines;
+    ld.g.s0 = 1;
+    const MixAccum st{tb, items, item0, synth, l0, a.pitch, sums, tsz};
     for (int z = 0; z < G; ++z) {
-        const float2* src = work + (long long)z * H;
-        for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-            int t = idx % T, i = idx / T, l = l0 + t;
-            a[t * npad + i] = l < nlines ? src[l + (long long)i * si] : make_float2(0.f, 0.f);
-        }
-        __syncthreads();
-        float2* r = fft_tile(a, b, T, sh, npad, tw, false);
-        const NSItem it = items[item0 + z];
-#pragma unroll
-        for (int e = 0; e < kAccMax; ++e) {
-            int idx = threadIdx.x + e * blockDim.x;
-            if (idx < total) {
-                int t = idx % T, i = idx / T, l = l0 + t;
-                if (l < nlines) {
-                    int k1 = l % tb.h1, k2 = l / tb.h1;
-                    float m = ns_mask(tb, it, k1, k2, i, l + (long long)i * si, synth != 0);
-                    float2 v = c_scale(r[t * npad + i], m);
-                    // Kahan: y = v - c ; t = s + y ; c = (t - s) - y ; s = t
-                    float2 y = c_sub(v, c[e]);
-                    float2 tt = c_add(s[e], y);
-                    c[e] = c_sub(c_sub(tt, s[e]), y);
-                    s[e] = tt;
-                }
-            }
-        }
-        __syncthreads();
+        mix_pass<false, BIG>(ld, st, a, tile, tile + tsz, tile + 2 * tsz, z);
+        __syncthreads();   // the tile is reused by the next item
     }
-#pragma unroll
-    for (int e = 0; e < kAccMax; ++e) {
-        int idx = threadIdx.x + e * blockDim.x;
-        if (idx < total) {
-            int t = idx % T, i = idx / T, l = l0 + t;
-            if (l < nlines) {
-                acc[l + (long long)i * si] = s[e];
-                comp[l + (long long)i * si] = c[e];
-            }
+    for (int it = threadIdx.x; it < n << a.lg; it += blockDim.x) {
+        const int t = it & (LP - 1), i = it >> a.lg;
+        if (l0 + t < a.nlines) {
+            acc[l0 + t + i * si] = sums[t * a.pitch + i];
+            comp[l0 + t + i * si] = sums[tsz + t * a.pitch + i];
         }
     }
 }
@@ -191,32 +172,68 @@ static void launch_accum_reg(const float2* W, long long H, int nz, const NSMaskT
 
 // ── set-up ───────────────────────────────────────────────────────────────────
 
-static std::vector<int> factorize(int n) {
-    std::vector<int> f;
-    for (int r : {8, 4, 2, 3, 5}) {
-        while (n % r == 0) {
-            f.push_back(r);
-            n /= r;
+// Fewest radices of the mixed-radix pass whose product is n, all but the last
+// (and the first, unless a large prime precedes them) from the middle set;
+// among those the smallest sum.
+static bool mix_search(int n, bool first, int left, std::vector<int>& cur, std::vector<int>& best) {
+    static const int middle[] = {19, 17, 16, 13, 11, 9, 8, 7, 5, 4, 3, 2};
+    auto sum = [](const std::vector<int>& v) {
+        int s = 0;
+        for (int r : v) s += r;
+        return s;
+    };
+    if (n <= 20) {
+        cur.push_back(n);
+        if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && sum(cur) < sum(best))) best = cur;
+        cur.pop_back();
+    }
+    if (left <= 1 || n == 1) return !best.empty();
+    auto take = [&](int r) {
+        if (n % r != 0 || n == r) return;
+        cur.push_back(r);
+        mix_search(n / r, false, left - 1, cur, best);
+        cur.pop_back();
+    };
+    if (first) {
+        for (int r = 20; r >= 2; --r) take(r);
+    } else {
+        for (int r : middle) take(r);
+    }
+    return !best.empty();
+}
+
+static MixSchedule mix_schedule(int n) {
+    std::vector<int> R;
+    int rest = n;
+    for (int p = 23; p <= rest; p += 2) {
+        bool prime = true;
+        for (int d = 3; d * d <= p; d += 2) prime = prime && p % d != 0;
+        while (prime && rest % p == 0) {
+            R.push_back(p);
+            rest /= p;
         }
     }
-    for (int p = 7; n > 1; p += 2) {
-        while (n % p == 0) {
-            f.push_back(p);
-            n /= p;
-        }
+    const size_t nbig = R.size();
+    if (rest > 1 || nbig != 1) {
+        std::vector<int> cur, best;
+        for (int steps = 1; steps + (int)nbig <= kMixMaxSteps && !mix_search(rest, nbig == 0, steps, cur, best); ++steps)
+            cur.clear();
+        if (best.empty()) throw ArgError("FFT length has too many factors");
+        R.insert(R.end(), best.begin(), best.end());
     }
-    return f;
+    MixSchedule m;
+    m.n = n;
+    m.ns = (int)R.size();
+    for (int s = 0; s < m.ns; ++s) m.R[s] = R[s];
+    return m;
 }
 
 FFTLen* get_fft(std::map<int, std::unique_ptr<FFTLen>>& cache, int n) {
     auto it = cache.find(n);
     if (it != cache.end()) return it->second.get();
     std::unique_ptr<FFTLen> f(new FFTLen);
-    std::vector<int> r = factorize(n);
-    if ((int)r.size() > kMaxStages) throw ArgError("FFT length has too many factors");
     f->sh.n = n;
-    f->sh.nstages = (int)r.size();
-    for (size_t i = 0; i < r.size(); ++i) f->sh.radix[i] = r[i];
+    f->mix = mix_schedule(n);
     std::vector<float2> tw(n);
     for (int t = 0; t < n; ++t) {
         // e^{-2 pi i t/n} designed in float64
@@ -226,6 +243,22 @@ FFTLen* get_fft(std::map<int, std::unique_ptr<FFTLen>>& cache, int n) {
     f->tw.alloc(sizeof(float2) * n);
     cuda_check(cudaMemcpy(f->tw.p, tw.data(), sizeof(float2) * n, cudaMemcpyHostToDevice), "twiddle upload");
     f->sh.tw = f->tw.as<float2>();
+    if (f->mix.ns > 2) {
+        // block e = (m_1, ..., m_{s-1}), the last digit fastest, holds the outputs from m_1 + R_1 (m_2 + ...)
+        const int nb = n / f->mix.R[f->mix.ns - 1];
+        std::vector<unsigned short> rev(nb);
+        for (int e = 0; e < nb; ++e) {
+            int q = e, k = 0;
+            for (int s = f->mix.ns - 2; s >= 0; --s) {
+                k = k * f->mix.R[s] + q % f->mix.R[s];
+                q /= f->mix.R[s];
+            }
+            rev[e] = (unsigned short)k;
+        }
+        f->rev.alloc(sizeof(unsigned short) * nb);
+        cuda_check(cudaMemcpy(f->rev.p, rev.data(), sizeof(unsigned short) * nb, cudaMemcpyHostToDevice),
+                   "digit table upload");
+    }
     FFTLen* raw = f.get();
     cache[n] = std::move(f);
     return raw;
@@ -403,13 +436,8 @@ void pass_r2c(NSPlan& P, const float* src, ZMap zin, int es, float2* dst, long l
     Lines gout = axis_lines(hg.d, 0);
     ZMap zo;
     zo.zstride = dst_zstride;
-    int pairs = (gin.nlines + 1) / 2;
-    if (launch_reg<false>(f->sh.n, RLoadRPair{src, zin, gin, es}, RStoreHalfPair{dst, zo, gout, f->sh.n}, f->sh.tw,
-                          pairs, nz, false, st, "ns_r2c_axis1"))
-        return;
-    LoadRPair ld{src, zin, gin, es};
-    StoreHalfPair sto{dst, zo, gout};
-    launch_pass(ld, sto, f->sh, pairs, nz, false, st, "ns_r2c_axis1");
+    launch_line<false>(*f, RLoadRPair{src, zin, gin, es}, RStoreHalfPair{dst, zo, gout, f->sh.n},
+                       (gin.nlines + 1) / 2, nz, false, st, "ns_r2c_axis1");
 }
 
 // C2R along axis 1 of nz spectra into nz real volumes, scaled.
@@ -421,13 +449,8 @@ void pass_c2r(NSPlan& P, const float2* src, long long src_zstride, float* dst, Z
     Lines gout = axis_lines(P.dims, 0);
     ZMap zi;
     zi.zstride = src_zstride;
-    int pairs = (gout.nlines + 1) / 2;
-    if (launch_reg<true>(f->sh.n, RLoadHPair{src, zi, gin, f->sh.n}, RStoreRPair{dst, zout, gout, es, scale},
-                         f->sh.tw, pairs, nz, false, st, "ns_c2r_axis1"))
-        return;
-    LoadHPair ld{src, zi, gin};
-    StoreRPair sto{dst, zout, gout, es, scale};
-    launch_pass(ld, sto, f->sh, pairs, nz, true, st, "ns_c2r_axis1");
+    launch_line<true>(*f, RLoadHPair{src, zi, gin, f->sh.n}, RStoreRPair{dst, zout, gout, es, scale},
+                      (gout.nlines + 1) / 2, nz, false, st, "ns_c2r_axis1");
 }
 
 // Complex FFT along axis a (1 or 2, 0-based) of nz spectra.
@@ -440,14 +463,10 @@ void pass_c2c(NSPlan& P, const float2* src, float2* dst, long long zstride, int 
     zm.zstride = zstride;
     const char* tag = axis == 1 ? "ns_c2c_axis2" : "ns_c2c_axis3";
     bool tf = g.si != 1;
-    bool done = inv ? launch_reg<true>(f->sh.n, RLoadC{src, zm, g}, RStoreC{dst, zm, g}, f->sh.tw, g.nlines, nz, tf,
-                                       st, tag)
-                    : launch_reg<false>(f->sh.n, RLoadC{src, zm, g}, RStoreC{dst, zm, g}, f->sh.tw, g.nlines, nz,
-                                        tf, st, tag);
-    if (done) return;
-    LoadC ld{src, zm, g, 1.f};
-    StoreC sto{dst, zm, g, 1.f};
-    launch_pass(ld, sto, f->sh, g.nlines, nz, inv, st, tag);
+    if (inv)
+        launch_line<true>(*f, RLoadC{src, zm, g}, RStoreC{dst, zm, g}, g.nlines, nz, tf, st, tag);
+    else
+        launch_line<false>(*f, RLoadC{src, zm, g}, RStoreC{dst, zm, g}, g.nlines, nz, tf, st, tag);
 }
 
 void rfft3(NSPlan& P, const float* x, int es, float2* X, cudaStream_t st) {
@@ -473,12 +492,8 @@ void analyze_items(NSPlan& P, const float2* X, float* cbase, ZMap zc, int es, in
     Lines g3 = axis_lines(hg.d, 2);
     ZMap zw;
     zw.zstride = P.H;
-    if (!launch_reg<true>(f3->sh.n, RLoadNSMask{X, P.tb, P.items.as<NSItem>(), i0, synth_masks ? 1 : 0},
-                          RStoreC{W, zw, g3}, f3->sh.tw, g3.nlines, nz, true, st, "ns_mask_axis3")) {
-        LoadNSMask ld{X, P.tb, P.items.as<NSItem>(), i0, synth_masks ? 1 : 0};
-        StoreC sto{W, zw, g3, 1.f};
-        launch_pass(ld, sto, f3->sh, g3.nlines, nz, true, st, "ns_mask_axis3");
-    }
+    launch_line<true>(*f3, RLoadNSMask{X, P.tb, P.items.as<NSItem>(), i0, synth_masks ? 1 : 0}, RStoreC{W, zw, g3}, g3.nlines, nz,
+                      true, st, "ns_mask_axis3");
     pass_c2c(P, W, W, P.H, 1, true, nz, st);
     pass_c2r(P, W, P.H, cbase, zc, es, 1.0f / (float)P.N, nz, st);
 }
@@ -512,25 +527,22 @@ void accum_items(NSPlan& P, int i0, int nz, bool analysis_masks, float2* acc, fl
             case 256: launch_accum_reg<256>(W, P.H, nz, P.tb, it, i0, sy, acc, comp, init, f3->sh.tw, nl, st); return;
         }
     }
-    int T = pass_tile(n);
-    while (T > 1 && T * n > kAccMax * 256) --T;
-    if (T * n > kAccMax * 256) throw ArgError("axis 3 is too long for the accumulating pass of this library");
-    int npad = n + 1;
-    size_t smem = pass_smem_bytes(n, T);
-    static bool configured = false;
-    if (!configured) {
-        cuda_check(cudaFuncSetAttribute(ns_accum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024),
+    if (n > kAccMaxLine) throw ArgError("axis 3 is too long for the accumulating pass of this library");
+    const bool big = f3->mix.R[0] > 20;
+    MixArgs a = mix_args(*f3, P.h1 * P.dims[1], true, false, 2 * sizeof(float2) * (n + 1));
+    const size_t smem = mix_smem_bytes(a.sc, a.lg, a.pitch, false) + 2 * sizeof(float2) * ((size_t)a.pitch << a.lg);
+    auto kern = big ? ns_accum_mix_kernel<true> : ns_accum_mix_kernel<false>;
+    static bool configured[2] = {false, false};
+    if (!configured[big]) {
+        cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
                    "cudaFuncSetAttribute");
-        configured = true;
+        configured[big] = true;
     }
-    int nlines = P.h1 * P.dims[1];
-    dim3 grid((nlines + T - 1) / T);
     int tok = prof_begin("ns_accum_axis3", st);
-    ns_accum_kernel<<<grid, 256, smem, st>>>(W, P.H, nz, P.tb, P.items.as<NSItem>(), i0,
-                                             analysis_masks ? 0 : 1, acc, comp, init ? 1 : 0,
-                                             f3->sh, T, npad);
+    kern<<<(a.nlines + (1 << a.lg) - 1) >> a.lg, mix_threads(a), smem, st>>>(
+        W, P.H, nz, P.tb, P.items.as<NSItem>(), i0, analysis_masks ? 0 : 1, acc, comp, init ? 1 : 0, a);
     prof_end(tok, st);
-    cuda_check(cudaGetLastError(), "ns_accum_kernel launch");
+    cuda_check(cudaGetLastError(), "ns_accum_mix_kernel launch");
 }
 
 void synth_items(NSPlan& P, const float* cbase, ZMap zc, int es, int i0, int nz, bool analysis_masks, float2* acc,
@@ -685,12 +697,8 @@ void ns_line_denoise_items(NSPlan& P, const float2* X, int i0, int nz, const flo
     Lines g3 = axis_lines(hg.d, 2);
     ZMap zw;
     zw.zstride = P.H;
-    if (!launch_reg<true>(f3->sh.n, RLoadNSMask{X, P.tb, P.items.as<NSItem>(), i0, 0}, RStoreC{W, zw, g3},
-                          f3->sh.tw, g3.nlines, nz, true, st, "ns_mask_axis3")) {
-        LoadNSMask ld{X, P.tb, P.items.as<NSItem>(), i0, 0};
-        StoreC sto{W, zw, g3, 1.f};
-        launch_pass(ld, sto, f3->sh, g3.nlines, nz, true, st, "ns_mask_axis3");
-    }
+    launch_line<true>(*f3, RLoadNSMask{X, P.tb, P.items.as<NSItem>(), i0, 0}, RStoreC{W, zw, g3}, g3.nlines, nz,
+                      true, st, "ns_mask_axis3");
     pass_c2c(P, W, W, P.H, 1, true, nz, st);
     FFTLen* f1 = get_fft(P.ffts, P.dims[0]);
     const Lines gh = axis_lines(hg.d, 0);

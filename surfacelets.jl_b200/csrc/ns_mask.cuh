@@ -3,65 +3,20 @@
 // by the NS drivers.
 #pragma once
 
-#include "passes.cuh"
+#include "mixpass.cuh"
 #include "plan.h"
 #include "regpass.cuh"
 
 namespace sfl {
 
-// Mask of item `it` at rfft-grid point (k1, k2, k3), linear index q.  synth
-// selects the synthesis mask, which is B_j alone when the bank is not tight
-// (src/transforms/ns_surfacelet.jl:226-227, 237-238).  The group factor
-// B_j hg_i comes from a float64-designed table; the wedge planes are
-// square-rooted in float64 too, so only well-conditioned float32 products
-// remain here.
-__device__ __forceinline__ float ns_mask(const NSMaskTables& tb, const NSItem& it, int k1, int k2, int k3,
-                                         long long q, bool synth) {
-    if (it.kind == 1) {
-        // lowpass a1 a2 a3: src/transforms/ns_surfacelet.jl:358-371
-        const float* v = tb.vec;
-        return v[tb.low_off[0] + k1] * v[tb.low_off[1] + k2] * v[tb.low_off[2] + k3];
-    }
-    if (synth && !tb.tight) return tb.Bl[(long long)it.lv * tb.H + q];
-    float G = tb.G[(long long)it.g * tb.H + q];
-    // wedge planes: src/transforms/ns_surfacelet.jl:376-427
-    int kk[3] = {k1, k2, k3};
-    float wa = tb.planes[it.wa_off + kk[it.wa_lo] + it.wa_dlo * kk[it.wa_hi]];
-    float wb = tb.planes[it.wb_off + kk[it.wb_lo] + it.wb_dlo * kk[it.wb_hi]];
-    return (G * wa) * wb;
-}
-
-// Pass-3 load of the analysis: lines along axis 3 of X, times the mask of
-// item z.  Line l = (k1, k2) with k1 fastest.
-struct LoadNSMask {
-    const float2* X;
-    NSMaskTables tb;
-    const NSItem* items;
-    int item0;
-    int synth;
-    __device__ __forceinline__ void operator()(float2* tile, int npad, int n, int l0, int T, int z) const {
-        const NSItem it = items[item0 + z];
-        const int nlines = tb.h1 * tb.n2;
-        const long long si = (long long)tb.h1 * tb.n2;
-        const int total = T * n;
-        for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-            int t = idx % T;
-            int i = idx / T;
-            int l = l0 + t;
-            float2 v = make_float2(0.f, 0.f);
-            if (l < nlines) {
-                int k1 = l % tb.h1, k2 = l / tb.h1;
-                long long q = l + (long long)i * si;
-                v = c_scale(X[q], ns_mask(tb, it, k1, k2, i, q, synth != 0));
-            }
-            tile[t * npad + i] = v;
-        }
-    }
-};
-
 // Per-line mask context of an NS item for lines along axis 3 (line l =
 // (k1, k2), element k3): mask(k3) = m[k3 * si] * wa(k3) * wb(k3), each plane
-// either constant along the line or stepping with k3.
+// either constant along the line or stepping with k3.  The group factor
+// B_j hg_i comes from a float64-designed table and the wedge planes are
+// square-rooted in float64 too (src/transforms/ns_surfacelet.jl:376-427), so
+// only well-conditioned float32 products remain; the lowpass is a1 a2 a3
+// (:358-371), and the synthesis mask of a bank that is not tight B_j alone
+// (:226-227, 237-238).
 struct NSMaskLine {
     const float* m;       // group table (or level bandpass) at the line's first point
     const float* wa;

@@ -71,6 +71,8 @@ struct DevMem {
 struct FFTLen {
     FFTShape sh;
     DevMem tw;
+    MixSchedule mix;   // lengths without a compile-time register pass
+    DevMem rev;        // output index of each block of the mixed schedule's last step (unsigned short)
 };
 
 // Per-subband descriptor of the NS cascade (device copy in NSPlan::items).

@@ -134,17 +134,31 @@ __device__ __forceinline__ void RegDft<R, INV>::run(float2 (&v)[R]) {
     constexpr int A = SplitOf<R>::A;
     constexpr CxTwTable<R, INV> tw{};
     if constexpr (B == R) {
-        // direct DFT of a prime size
-        float2 out[R];
+        // odd prime size: with s_r = v_r + v_{R-r} and d_r = -i (v_r - v_{R-r}) (formed rotated by scalar
+        // subtractions), bins m and R - m are C +- D, C = v_0 + sum s_r cos, D = sum d_r sin (2 pi r m / R)
+        constexpr int H = (R - 1) / 2;
+        float2 sp[H], dp[H];
+        float2 z = v[0];
 #pragma unroll
-        for (int m = 0; m < R; ++m) {
-            float2 acc = v[0];
-#pragma unroll
-            for (int r = 1; r < R; ++r) acc = c_add(acc, c_mul(v[r], tw.v[(r * m) % R]));
-            out[m] = acc;
+        for (int r = 1; r <= H; ++r) {
+            sp[r - 1] = c_add(v[r], v[R - r]);
+            dp[r - 1] = make_float2(v[r].y - v[R - r].y, v[R - r].x - v[r].x);
+            z = c_add(z, sp[r - 1]);
         }
 #pragma unroll
-        for (int m = 0; m < R; ++m) v[m] = out[m];
+        for (int m = 1; m <= H; ++m) {
+            float2 C = v[0], D = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int r = 1; r <= H; ++r) {
+                const int e = (r * m) % R;
+                C = c_fma(sp[r - 1], tw.v[e].x, C);
+                // tw holds -sin (forward) or +sin (inverse)
+                D = r == 1 ? c_scale(dp[0], -tw.v[e].y) : c_fma(dp[r - 1], -tw.v[e].y, D);
+            }
+            v[m] = c_add(C, D);
+            v[R - m] = c_sub(C, D);
+        }
+        v[0] = z;
     } else {
         // n = a + A b, k = kb + B ka: inner DFT_B over b, twiddle w_R^{a kb}, outer DFT_A over a
         float2 t[R];
