@@ -406,7 +406,8 @@ void ns_plan_init(NSPlan& P, const sfl_ns_params& p, const int dims[3], int dtyp
 void ns_alloc_scratch(NSPlan& P) {
     const long long spec = P.slab ? P.SP : P.H;
     P.X.alloc(sizeof(float2) * spec * P.nch);
-    P.work.alloc(sizeof(float2) * spec * P.group * (P.slab ? P.nch : 1));
+    P.slots = P.slab ? ns_slab_slots(P) : P.group;
+    P.work.alloc(sizeof(float2) * spec * P.slots * (P.slab ? P.nch : 1));
     if (P.slab) {
         P.acc.alloc(sizeof(float2) * spec * P.nch);
         P.comp.alloc(sizeof(float2) * spec * P.nch);
@@ -662,7 +663,7 @@ void ns_accumulate_range(NSPlan& P, const float* vol, ZMap vz, int es, int i0, i
 
 void ns_stage_range(NSPlan& P, const float* vol, ZMap vz, int es, int i0, int nz, int slot0, int nch,
                     cudaStream_t st) {
-    if (slot0 < 0 || slot0 + nz > P.group) throw ArgError("work slots out of range");
+    if (slot0 < 0 || slot0 + nz > P.slots) throw ArgError("work slots out of range");
     if (P.slab) {
         ns_slab_stage_items(P, vol, vz, es, i0, nz, slot0, nch, st);
     } else {

@@ -77,9 +77,9 @@ void need_bf16_path(const NSPlan& P) {
 }
 
 void ensure_band(NSPlan& P) {
-    const size_t need = sizeof(float) * (size_t)P.N * P.group;
+    const size_t need = sizeof(float) * (size_t)P.N * P.slots;
     if (P.band.bytes < need) P.band.alloc(need);
-    if (P.maxbits.bytes < sizeof(unsigned) * (size_t)P.group) P.maxbits.alloc(sizeof(unsigned) * P.group);
+    if (P.maxbits.bytes < sizeof(unsigned) * (size_t)P.slots) P.maxbits.alloc(sizeof(unsigned) * P.slots);
 }
 
 }  // namespace

@@ -36,7 +36,7 @@ void ns_denoise(NSPlan& P, const float* x, float* y, const float* tau, cudaStrea
     ns_acc_clear(P, A, K, st);
     const bool fused_lines = !P.slab && ns_line_shrink_supported(P);
     if (!P.slab && !fused_lines) {
-        const size_t need = sizeof(float) * (size_t)P.N * P.group;
+        const size_t need = sizeof(float) * (size_t)P.N * P.slots;
         if (P.band.bytes < need) P.band.alloc(need);
     }
     ZMap vz;

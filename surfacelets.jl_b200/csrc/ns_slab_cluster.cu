@@ -194,7 +194,9 @@ struct ClusterCtx {
     float2* S1;
     uint64_t* bar;
     uint32_t phase = 0;
-    int rank, r0, rn;
+    int rank, r0;
+    // own rows inside a box of nk1 rows
+    __device__ __forceinline__ int rows(int nk1) const { return min(rank == 0 ? C::R : C::H1 - C::R, nk1 - r0); }
     __device__ __forceinline__ ClusterCtx(float2* sm, const SlabArgs& a) {
         cg::cluster_group cl = cg::this_cluster();
         twA = sm;
@@ -205,7 +207,6 @@ struct ClusterCtx {
         S0 = cl.map_shared_rank(S, 0);
         S1 = cl.map_shared_rank(S, 1);
         r0 = rank * C::R;
-        rn = min(rank == 0 ? C::R : C::H1 - C::R, a.nk1 - r0);
         bar = reinterpret_cast<uint64_t*>(X + C::LINES * NA);
         if (threadIdx.x == 0) {
             mbar_init(bar, 1);
@@ -217,7 +218,7 @@ struct ClusterCtx {
 };
 
 template <int NA, int NB, int ES>
-__global__ void __launch_bounds__(kSlabThreads, 1) ns_slab_cluster_inv_kernel(SlabArgs a) {
+__global__ void __launch_bounds__(kSlabThreads, 1) ns_slab_cluster_inv_kernel(const __grid_constant__ SlabArgs a) {
     using C = ClusterSlab<NA, NB>;
     using LA = SlabLine<NA>;
     extern __shared__ float2 sm[];
@@ -227,23 +228,25 @@ __global__ void __launch_bounds__(kSlabThreads, 1) ns_slab_cluster_inv_kernel(Sl
     constexpr long long PLANE = (long long)NA * NB;
     const int nclusters = gridDim.x / kClusterCTAs;
     for (int u = blockIdx.x / kClusterCTAs; u < a.units; u += nclusters) {
-        const int per = a.nzc * a.n3;
+        const int per = a.ck.nz * a.n3;
         const int ch = u / per, ur = u - ch * per;
         const int z = ur / a.n3, s3 = ur - z * a.n3;
+        const int nk1 = a.ck.item[z].nk1, nk2 = a.ck.item[z].nk2, b2 = a.ck.item[z].b2;
+        const int rn = cx.rows(nk1);
         const float2* src = a.spec + ch * a.spec_chstride + z * a.spec_zstride + (long long)s3 * (C::P1 * NB);
-        load_rows<NB, C::P1, C::PL>(cx.S, src, cx.r0, cx.rn, a.nk2, a.b2, cx.bar, cx.phase, a.status);
-        rows_fft<NB, C::PL, true>(cx.S, cx.twB, cx.rn, a.nk2, a.b2, warp, lane);
+        load_rows<NB, C::P1, C::PL>(cx.S, src, cx.r0, rn, nk2, b2, cx.bar, cx.phase, a.status);
+        rows_fft<NB, C::PL, true>(cx.S, cx.twB, rn, nk2, b2, warp, lane);
         cluster_barrier();   // both halves of every column are final
         {
             const int p = lane & (LA::N2 - 1), s = pair_subline<NA>(lane / LA::N2);
-            float* out = a.vol + ch + a.vz.off(z) + (long long)s3 * PLANE * ES;
+            float* out = a.vol + ch + a.vol_off(z) + (long long)s3 * PLANE * ES;
             float2* xs = cx.X + (warp * LA::LPW + s) * NA;
             for (int base = 0; base < C::PAIRS; base += LA::LPR) {
                 const int lo = base + warp * LA::LPW + s;   // own pair index
                 const bool valid = lo < C::PAIRS;
                 const int l = cx.rank * C::PAIRS + (valid ? lo : 0);
                 float2 v[LA::N1];
-                load_pair<NA, NB>(v, cx.S0, cx.S1, l, p, valid, a.nk1);
+                load_pair<NA, NB>(v, cx.S0, cx.S1, l, p, valid, nk1);
                 warp_line_fft<NA, true, 1>(v, p, valid, cx.twA, xs);
                 if (valid) {
                     float* oa = out + (long long)(2 * l) * NA * ES;
@@ -266,7 +269,7 @@ __global__ void __launch_bounds__(kSlabThreads, 1) ns_slab_cluster_inv_kernel(Sl
 }
 
 template <int NA, int NB, int ES>
-__global__ void __launch_bounds__(kSlabThreads, 1) ns_slab_cluster_fwd_kernel(SlabArgs a) {
+__global__ void __launch_bounds__(kSlabThreads, 1) ns_slab_cluster_fwd_kernel(const __grid_constant__ SlabArgs a) {
     using C = ClusterSlab<NA, NB>;
     using LA = SlabLine<NA>;
     extern __shared__ float2 sm[];
@@ -276,12 +279,14 @@ __global__ void __launch_bounds__(kSlabThreads, 1) ns_slab_cluster_fwd_kernel(Sl
     constexpr long long PLANE = (long long)NA * NB;
     const int nclusters = gridDim.x / kClusterCTAs;
     for (int u = blockIdx.x / kClusterCTAs; u < a.units; u += nclusters) {
-        const int per = a.nzc * a.n3;
+        const int per = a.ck.nz * a.n3;
         const int ch = u / per, ur = u - ch * per;
         const int z = ur / a.n3, s3 = ur - z * a.n3;
+        const int nk1 = a.ck.item[z].nk1, nk2 = a.ck.item[z].nk2, b2 = a.ck.item[z].b2;
+        const int rn = cx.rows(nk1);
         {
             const int p = lane & (LA::N2 - 1), s = pair_subline<NA>(lane / LA::N2);
-            const float* in = a.vol + ch + a.vz.off(z) + (long long)s3 * PLANE * ES;
+            const float* in = a.vol + ch + a.vol_off(z) + (long long)s3 * PLANE * ES;
             float2* xs = cx.X + (warp * LA::LPW + s) * NA;
             for (int base = 0; base < C::PAIRS; base += LA::LPR) {
                 const int lo = base + warp * LA::LPW + s;
@@ -303,21 +308,21 @@ __global__ void __launch_bounds__(kSlabThreads, 1) ns_slab_cluster_fwd_kernel(Sl
                         for (int k = 0; k < LA::N2; ++k) xs[(p + LA::N2 * j) + LA::N1 * k] = v[j * LA::N2 + k];
                 }
                 __syncwarp();
-                unpack_pair<NA, NB>(xs, cx.S0, cx.S1, l, p, valid, a.nk1);
+                unpack_pair<NA, NB>(xs, cx.S0, cx.S1, l, p, valid, nk1);
                 __syncwarp();   // the exchange slots are reused by the next pair
             }
         }
         cluster_barrier();   // every row is complete in its CTA
-        rows_fft<NB, C::PL, false>(cx.S, cx.twB, cx.rn, a.nk2, a.b2, warp, lane);
+        rows_fft<NB, C::PL, false>(cx.S, cx.twB, rn, nk2, b2, warp, lane);
         __syncthreads();
         float2* dst = a.spec + ch * a.spec_chstride + z * a.spec_zstride + (long long)s3 * (C::P1 * NB);
-        store_rows<NB, C::P1, C::PL>(dst, cx.S, cx.r0, cx.rn, a.nk2, a.b2);
+        store_rows<NB, C::P1, C::PL>(dst, cx.S, cx.r0, rn, nk2, b2);
         cluster_barrier();   // the rows are free for the peer's next unit
     }
 }
 
 template <int NA, int NB>
-__global__ void __launch_bounds__(kSlabThreads, 1) ns_slab_cluster_shrink_kernel(SlabArgs a) {
+__global__ void __launch_bounds__(kSlabThreads, 1) ns_slab_cluster_shrink_kernel(const __grid_constant__ SlabArgs a) {
     using C = ClusterSlab<NA, NB>;
     using LA = SlabLine<NA>;
     extern __shared__ float2 sm[];
@@ -326,13 +331,15 @@ __global__ void __launch_bounds__(kSlabThreads, 1) ns_slab_cluster_shrink_kernel
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nclusters = gridDim.x / kClusterCTAs;
     for (int u = blockIdx.x / kClusterCTAs; u < a.units; u += nclusters) {
-        const int per = a.nzc * a.n3;
+        const int per = a.ck.nz * a.n3;
         const int ch = u / per, ur = u - ch * per;
         const int z = ur / a.n3, s3 = ur - z * a.n3;
+        const int nk1 = a.ck.item[z].nk1, nk2 = a.ck.item[z].nk2, b2 = a.ck.item[z].b2;
+        const int rn = cx.rows(nk1);
         float2* slab = a.spec + ch * a.spec_chstride + z * a.spec_zstride + (long long)s3 * (C::P1 * NB);
-        const float tau = a.tau[a.items[a.item0 + z].s - 1];
-        load_rows<NB, C::P1, C::PL>(cx.S, slab, cx.r0, cx.rn, a.nk2, a.b2, cx.bar, cx.phase, a.status);
-        rows_fft<NB, C::PL, true>(cx.S, cx.twB, cx.rn, a.nk2, a.b2, warp, lane);
+        const float tau = a.tau[a.ck.item[z].s - 1];
+        load_rows<NB, C::P1, C::PL>(cx.S, slab, cx.r0, rn, nk2, b2, cx.bar, cx.phase, a.status);
+        rows_fft<NB, C::PL, true>(cx.S, cx.twB, rn, nk2, b2, warp, lane);
         cluster_barrier();
         {
             const int p = lane & (LA::N2 - 1), s = pair_subline<NA>(lane / LA::N2);
@@ -342,7 +349,7 @@ __global__ void __launch_bounds__(kSlabThreads, 1) ns_slab_cluster_shrink_kernel
                 const bool valid = lo < C::PAIRS;
                 const int l = cx.rank * C::PAIRS + (valid ? lo : 0);
                 float2 v[LA::N1];
-                load_pair<NA, NB>(v, cx.S0, cx.S1, l, p, valid, a.nk1);
+                load_pair<NA, NB>(v, cx.S0, cx.S1, l, p, valid, nk1);
                 warp_line_fft<NA, true, 1>(v, p, valid, cx.twA, xs);
                 if (valid) {
 #pragma unroll
@@ -366,14 +373,14 @@ __global__ void __launch_bounds__(kSlabThreads, 1) ns_slab_cluster_shrink_kernel
                         for (int k = 0; k < LA::N2; ++k) xs[(p + LA::N2 * j) + LA::N1 * k] = v[j * LA::N2 + k];
                 }
                 __syncwarp();
-                unpack_pair<NA, NB>(xs, cx.S0, cx.S1, l, p, valid, a.nk1);
+                unpack_pair<NA, NB>(xs, cx.S0, cx.S1, l, p, valid, nk1);
                 __syncwarp();
             }
         }
         cluster_barrier();   // every row holds the re-transformed columns
-        rows_fft<NB, C::PL, false>(cx.S, cx.twB, cx.rn, a.nk2, a.b2, warp, lane);
+        rows_fft<NB, C::PL, false>(cx.S, cx.twB, rn, nk2, b2, warp, lane);
         __syncthreads();
-        store_rows<NB, C::P1, C::PL>(slab, cx.S, cx.r0, cx.rn, a.nk2, a.b2);
+        store_rows<NB, C::P1, C::PL>(slab, cx.S, cx.r0, rn, nk2, b2);
         __syncthreads();   // own rows are reloaded by the next unit (the peer writes them only after the next barrier)
     }
 }
@@ -416,7 +423,6 @@ template <int NA, int NB>
 void launch_nn(int kind, const SlabArgs& a, int sms, cudaStream_t st, const char* tag) {
     using C = ClusterSlab<NA, NB>;
     if (a.P1 != C::P1) throw ArgError("slab pitch mismatch");
-    if (a.nk1 > C::H1 || a.nk2 > NB) throw ArgError("slab box out of range");
     if (kind == 1) {
         if (a.es == 1)
             launch_cluster<1, NA, NB, 1>(a, sms, st, tag);

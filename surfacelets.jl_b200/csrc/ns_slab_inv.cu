@@ -1,0 +1,10 @@
+// The inverse slab pass of every compile-time slab size.
+#include "ns_slab_pass.cuh"
+
+namespace sfl {
+
+void launch_slab_inv(int na, int nb, const SlabArgs& a, int sms, size_t smem, cudaStream_t st, const char* tag) {
+    launch_slab_kind<1>(na, nb, a, sms, smem, st, tag);
+}
+
+}  // namespace sfl

@@ -129,6 +129,7 @@ struct NSPlan {
     int nch = 1;          // 1 real, 2 complex
     bool ndfb = false;    // the standalone directional bank (no pyramid, no lowpass)
     int group = 8;
+    int slots = 8;        // work spectra: subbands in flight per launch (the slab pipeline's chunks)
     int ipc = 0;          // subbands a CTA of the slab axis-3 analysis pass takes (1, 2, 4, 8; 0: the default, mask_ipc)
     std::vector<NSItem> items_host;   // streaming / item order: directional ascending, then lowpass
     DevMem items;
@@ -191,6 +192,7 @@ bool ns_slab_supported(int n1, int n2, int n3);
 // larger CTAs over filling the GPU alone.
 void ns_set_concurrent(bool on);
 void ns_use_slabs(NSPlan& P);
+int ns_slab_slots(const NSPlan& P);
 NSBox ns_make_box(int nk1, int b2, int n2);
 NSBox ns_table_box(const std::vector<double>& g, int h1, int n2, int n3);
 void ns_alloc_scratch(NSPlan& P);

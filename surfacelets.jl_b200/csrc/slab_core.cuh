@@ -13,24 +13,55 @@ constexpr int kSlabThreads = 512;
 constexpr int kSlabWarps = kSlabThreads / 32;
 constexpr size_t kSlabSmemOneCta = 227 * 1024;   // the most one CTA may hold
 
+// A chunk: the subbands of one pair of launches (an axis-3 pass and a slab
+// pass), consecutive items in streaming order, as segments of one mask group
+// each.  Passed to the kernels by value, so that what a CTA does with an item
+// is read from constant memory (the device copies of the items cost a chain of
+// dependent loads per item: the synthesis axis-3 pass of a small chunk spent
+// more time on those than on its FFTs).  The work slot of an item is its
+// position in the chunk.
+constexpr int kChunkItems = 64, kChunkSegs = 24;
+struct ChunkItem {
+    int s;                        // 1-based subband index
+    int wa_off, wb_off;           // float offsets of the two wedge planes
+    short wa_dlo, wb_dlo;         // their extents along the first axis
+    signed char wa_lo, wa_hi, wb_lo, wb_hi;   // their axes, 0-based
+    short nk1, nk2, b2;           // support box (NSBox)
+    short seg;
+};
+struct ChunkSeg {
+    int g, lv;                    // mask group (its table), pyramid level (its bandpass)
+    short i0, nz;                 // items [i0, i0 + nz) of the chunk
+    short nbq;                    // > 0: nbq plane-b wedges times whole rows of plane-a wedges constant along axis 3
+    short low;                    // the lowpass
+    short nk1, nk2, b2;           // support box
+    short pad;
+};
+struct Chunk {
+    int nz, nseg;
+    ChunkSeg seg[kChunkSegs];
+    ChunkItem item[kChunkItems];
+};
+
 struct SlabArgs {
     float2* spec;            // padded spectra, item z at spec + z * spec_zstride
     long long spec_zstride;
-    float* vol;              // real volumes (element stride es), item z at vol + vz.off(z)
-    ZMap vz;
+    float* vol;              // real volumes (element stride es): item z's at vol + z * vol_zstride, or, with
+    long long vol_zstride;   // vol_sub_stride, at vol + (s - 1) vol_sub_stride of its subband s
+    long long vol_sub_stride;
     int es;
     float scale;             // applied to the C2R outputs
     int P1, n3;
-    int nk1, nk2, b2;        // box: rows k1 < nk1, columns as BoxMap
     int units;               // channels x items x n3
-    int nzc;                 // items a channel
     long long spec_chstride; // spectra: channel stride (the volume's channels are interleaved floats)
     const float2* twa;       // w_n1^k, k < n1 (float64-designed)
     const float2* twb;       // w_n2^k, k < n2
     const float* tau;        // shrink pass: threshold of subband s at tau[s - 1]
-    const NSItem* items;     // shrink pass: the launch's items, from item0
-    int item0;
     int* status;             // the plan's device status word (bounded waits record a timeout there)
+    Chunk ck;
+    __device__ __forceinline__ long long vol_off(int z) const {
+        return vol_sub_stride ? (long long)(ck.item[z].s - 1) * vol_sub_stride : z * vol_zstride;
+    }
 };
 
 template <int N>
@@ -144,6 +175,11 @@ __device__ __forceinline__ int pair_subline(int s) {
     if (SlabLine<N>::LPW == 4) return s == 1 ? 2 : (s == 2 ? 1 : s);
     return s;
 }
+
+// The slab passes of the compile-time sizes (ns_slab_pass.cuh, one CTA a slab).
+void launch_slab_fwd(int na, int nb, const SlabArgs& a, int sms, size_t smem, cudaStream_t st, const char* tag);
+void launch_slab_inv(int na, int nb, const SlabArgs& a, int sms, size_t smem, cudaStream_t st, const char* tag);
+void launch_slab_shrink(int na, int nb, const SlabArgs& a, int sms, size_t smem, cudaStream_t st, const char* tag);
 
 // Launches a slab pass of a size with a cluster kernel (ns_slab_cluster.cu).
 // KIND: 0 forward, 1 inverse, 2 the denoiser's shrink pass.  Returns false
