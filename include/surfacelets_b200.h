@@ -194,6 +194,9 @@ int sfl_plan_set_group(sfl_plan* plan, int32_t group);
  *     or 256, axis 3 of length 16, 32, 64, 96, 128, 160 or 256): a line pass
  *     along axis 3 plus one pass per axis-3 slab, skipping the zero rows and
  *     columns of band-limited masks.
+ *   MIXED (default for the other lengths whose slabs fit shared memory, about
+ *     216 x 216 and, with more room, odd and prime lengths too): the same two
+ *     passes on a mixed-radix FFT.
  *   LINES (default elsewhere): one line pass per axis.
  *   PLANES: retired (the plane-major pipeline was slower than SLABS at every
  *     size it supported); selecting it returns SFL_ERR_ARGUMENT.
@@ -201,6 +204,7 @@ int sfl_plan_set_group(sfl_plan* plan, int32_t group);
 #define SFL_PIPELINE_LINES 0
 #define SFL_PIPELINE_PLANES 1
 #define SFL_PIPELINE_SLABS 2
+#define SFL_PIPELINE_MIXED 3
 int sfl_plan_set_pipeline(sfl_plan* plan, int32_t pipeline);
 
 /* The plan's pipeline and group.  No counterpart in the reference. */

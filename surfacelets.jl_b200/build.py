@@ -46,7 +46,7 @@ def compile_one(src, force, verbose):
     return obj
 
 
-def build(force=False, jobs=8, verbose=False):
+def build(force=False, jobs=10, verbose=False):
     os.makedirs(OBJ, exist_ok=True)
     srcs = sources()
     with cf.ThreadPoolExecutor(max_workers=jobs) as ex:
@@ -63,7 +63,7 @@ def build(force=False, jobs=8, verbose=False):
 if __name__ == "__main__":
     ap = argparse.ArgumentParser()
     ap.add_argument("--force", action="store_true")
-    ap.add_argument("--jobs", type=int, default=8)
+    ap.add_argument("--jobs", type=int, default=10)
     ap.add_argument("--verbose", action="store_true", help="print ptxas register/smem usage")
     a = ap.parse_args()
     print(build(a.force, a.jobs, a.verbose))

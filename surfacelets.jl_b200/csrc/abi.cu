@@ -152,7 +152,7 @@ void ns_apply(sfl::NSPlan& N, int pipeline, int group, int ipc = -1) {
     cudaDeviceSynchronize();
     if (pipeline == SFL_PIPELINE_LINES) {
         if (N.slab) {
-            N.slab = false;
+            N.slab = N.mixed = false;
             sfl::ns_alloc_scratch(N);
         }
     } else if (pipeline == SFL_PIPELINE_PLANES) {
@@ -160,6 +160,8 @@ void ns_apply(sfl::NSPlan& N, int pipeline, int group, int ipc = -1) {
                             "supported");
     } else if (pipeline == SFL_PIPELINE_SLABS) {
         sfl::ns_use_slabs(N);
+    } else if (pipeline == SFL_PIPELINE_MIXED) {
+        sfl::ns_use_mixed(N);
     } else {
         throw sfl::ArgError("unknown pipeline " + std::to_string(pipeline));
     }
@@ -170,7 +172,7 @@ void ns_apply(sfl::NSPlan& N, int pipeline, int group, int ipc = -1) {
 }
 
 int ns_pipeline_of(const sfl::NSPlan& N) {
-    return N.slab ? SFL_PIPELINE_SLABS : SFL_PIPELINE_LINES;
+    return N.mixed ? SFL_PIPELINE_MIXED : (N.slab ? SFL_PIPELINE_SLABS : SFL_PIPELINE_LINES);
 }
 
 // Tuned (pipeline, group) per transform, size and element type, for the
@@ -613,6 +615,7 @@ int sfl_plan_autotune(sfl_plan* plan, const void* x, void* c, void* stream) {
             try {
                 std::vector<int> pipes;
                 if (sfl::ns_slab_supported(N.dims[0], N.dims[1], N.dims[2])) pipes.push_back(SFL_PIPELINE_SLABS);
+                if (sfl::ns_mix_slab_supported(N)) pipes.push_back(SFL_PIPELINE_MIXED);
                 pipes.push_back(SFL_PIPELINE_LINES);
                 // pipeline x group at the default tile, then the slab tile (subbands a CTA of the axis-3
                 // analysis pass) for the best group
@@ -625,7 +628,7 @@ int sfl_plan_autotune(sfl_plan* plan, const void* x, void* c, void* stream) {
                             pick = {pipe, g, 0};
                         }
                     }
-                if (pick.pipeline == SFL_PIPELINE_SLABS)
+                if (pick.pipeline != SFL_PIPELINE_LINES)
                     for (int ipc : {1, 2, 4}) {
                         const float ms = time_it(pick.pipeline, pick.group, ipc);
                         if (ms < best) {
@@ -1097,15 +1100,21 @@ int sfl_ns_accumulate_range(sfl_plan* plan, const void* c, int32_t first, int32_
         on_device(plan, [&] {
             for (int ch = 0; ch < N.nch; ++ch) {
                 float2* acc = static_cast<float2*>(A) + ch * E;
-                float2* comp = sfl::ns_comp_grid(N, ch);
+                float2* comp = sfl::ns_range_comp(N, ch);
                 if (clear) sfl::ns_acc_clear(N, acc, comp, as_stream(stream));
+                // with several accumulators the range goes through the plan's, then into A
+                const bool groups = N.slab && N.ngrp > 1;
+                float2* to = groups ? N.acc.as<float2>() + ch * E : acc;
+                float2* tc = groups ? sfl::ns_comp_grid(N, ch) : comp;
+                if (groups) sfl::ns_acc_clear(N, to, tc, as_stream(stream));
                 for (int i0 = first, i1; i0 < first + count; i0 = i1) {
                     i1 = std::min(sfl::ns_next_chunk(N, i0), first + count);
                     sfl::ZMap vz;
                     vz.zstride = N.N * N.nch;
                     const float* base = static_cast<const float*>(c) + (long long)(i0 - first) * N.N * N.nch + ch;
-                    sfl::ns_accumulate_range(N, base, vz, N.nch, i0, i1 - i0, false, acc, comp, as_stream(stream));
+                    sfl::ns_accumulate_range(N, base, vz, N.nch, i0, i1 - i0, false, to, tc, as_stream(stream));
                 }
+                if (groups) sfl::ns_merge_groups(N, ch, acc, comp, as_stream(stream));
             }
         });
         return SFL_OK;

@@ -13,7 +13,7 @@ struct FFTShape {
 };
 
 // Radices of the mixed-radix line pass (mixpass.cuh) of a length, in step
-// order: its large prime factors, then radices of at most 20.
+// order: its large prime factors, then radices of at most 16.
 constexpr int kMixMaxSteps = 8;
 struct MixSchedule {
     int n = 1;

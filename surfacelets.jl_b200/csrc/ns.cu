@@ -14,6 +14,7 @@
 // designed in float64: the group factor B_j hg_i on the rfft grid (one table
 // per scale and hourglass) and the wedge planes; M_s itself is never
 // materialized.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -54,31 +55,32 @@ template <bool BIG>
 __global__ void __launch_bounds__(256, 2) ns_accum_mix_kernel(const float2* __restrict__ work, long long H, int G,
                                                               NSMaskTables tb, const NSItem* __restrict__ items,
                                                               int item0, int synth, float2* acc, float2* comp, int init,
-                                                              MixArgs a) {
+                                                              const __grid_constant__ MixArgs a, int nlines, int lg) {
     extern __shared__ float2 smem[];
-    const int tsz = a.pitch << a.lg, LP = 1 << a.lg, l0 = blockIdx.x << a.lg, n = a.sc.n;
+    const int tsz = a.pitch << lg, LP = 1 << lg, l0 = blockIdx.x << lg, n = a.sc.n;
+    const MixTile g{l0, nlines, lg, 1};
     const long long si = (long long)tb.h1 * tb.n2;
     float2* sums = smem;
     float2* tile = smem + 2 * tsz;
-    for (int it = threadIdx.x; it < n << a.lg; it += blockDim.x) {
-        const int t = it & (LP - 1), i = it >> a.lg;
-        const bool have = !init && l0 + t < a.nlines;
+    for (int it = threadIdx.x; it < n << lg; it += blockDim.x) {
+        const int t = it & (LP - 1), i = it >> lg;
+        const bool have = !init && l0 + t < nlines;
         sums[t * a.pitch + i] = have ? acc[l0 + t + i * si] : make_float2(0.f, 0.f);
         sums[tsz + t * a.pitch + i] = have ? comp[l0 + t + i * si] : make_float2(0.f, 0.f);
     }
     RLoadC ld{work, ZMap{}, Lines{}};
     ld.zm.zstride = H;
     ld.g.si = si;
-    ld.g.B0 = a.nlines;
+    ld.g.B0 = nlines;
     ld.g.s0 = 1;
     const MixAccum st{tb, items, item0, synth, l0, a.pitch, sums, tsz};
     for (int z = 0; z < G; ++z) {
-        mix_pass<false, BIG>(ld, st, a, tile, tile + tsz, tile + 2 * tsz, z);
+        mix_pass<false, BIG>(ld, st, a, g, tile, tile + tsz, tile + 2 * tsz, z);
         __syncthreads();   // the tile is reused by the next item
     }
-    for (int it = threadIdx.x; it < n << a.lg; it += blockDim.x) {
-        const int t = it & (LP - 1), i = it >> a.lg;
-        if (l0 + t < a.nlines) {
+    for (int it = threadIdx.x; it < n << lg; it += blockDim.x) {
+        const int t = it & (LP - 1), i = it >> lg;
+        if (l0 + t < nlines) {
             acc[l0 + t + i * si] = sums[t * a.pitch + i];
             comp[l0 + t + i * si] = sums[tsz + t * a.pitch + i];
         }
@@ -176,13 +178,13 @@ static void launch_accum_reg(const float2* W, long long H, int nz, const NSMaskT
 // (and the first, unless a large prime precedes them) from the middle set;
 // among those the smallest sum.
 static bool mix_search(int n, bool first, int left, std::vector<int>& cur, std::vector<int>& best) {
-    static const int middle[] = {19, 17, 16, 13, 11, 9, 8, 7, 5, 4, 3, 2};
+    static const int middle[] = {13, 11, 8, 7, 5, 4, 3, 2};
     auto sum = [](const std::vector<int>& v) {
         int s = 0;
         for (int r : v) s += r;
         return s;
     };
-    if (n <= 20) {
+    if (n <= 16) {
         cur.push_back(n);
         if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && sum(cur) < sum(best))) best = cur;
         cur.pop_back();
@@ -195,7 +197,7 @@ static bool mix_search(int n, bool first, int left, std::vector<int>& cur, std::
         cur.pop_back();
     };
     if (first) {
-        for (int r = 20; r >= 2; --r) take(r);
+        for (int r = 16; r >= 2; --r) take(r);
     } else {
         for (int r : middle) take(r);
     }
@@ -205,7 +207,7 @@ static bool mix_search(int n, bool first, int left, std::vector<int>& cur, std::
 static MixSchedule mix_schedule(int n) {
     std::vector<int> R;
     int rest = n;
-    for (int p = 23; p <= rest; p += 2) {
+    for (int p = 17; p <= rest; p += 2) {
         bool prime = true;
         for (int d = 3; d * d <= p; d += 2) prime = prime && p % d != 0;
         while (prime && rest % p == 0) {
@@ -213,6 +215,7 @@ static MixSchedule mix_schedule(int n) {
             rest /= p;
         }
     }
+    std::reverse(R.begin(), R.end());   // the largest first: the passes size their weight table by R[0]
     const size_t nbig = R.size();
     if (rest > 1 || nbig != 1) {
         std::vector<int> cur, best;
@@ -399,6 +402,7 @@ void ns_plan_init(NSPlan& P, const sfl_ns_params& p, const int dims[3], int dtyp
     while (P.P1 % 4 != 2) ++P.P1;
     P.SP = (long long)P.P1 * dims[1] * dims[2];
     P.slab = ns_slab_supported(dims[0], dims[1], dims[2]);
+    if (!P.slab) P.slab = P.mixed = ns_mix_slab_supported(P);
     ns_alloc_scratch(P);
 }
 
@@ -408,9 +412,11 @@ void ns_alloc_scratch(NSPlan& P) {
     P.X.alloc(sizeof(float2) * spec * P.nch);
     P.slots = P.slab ? ns_slab_slots(P) : P.group;
     P.work.alloc(sizeof(float2) * spec * P.slots * (P.slab ? P.nch : 1));
+    P.ngrp = P.slab ? ns_slab_groups(P) : 1;
+    P.rcomp.alloc(P.ngrp > 1 ? sizeof(float2) * spec * P.nch : 0);
     if (P.slab) {
-        P.acc.alloc(sizeof(float2) * spec * P.nch);
-        P.comp.alloc(sizeof(float2) * spec * P.nch);
+        P.acc.alloc(sizeof(float2) * spec * P.nch * P.ngrp);
+        P.comp.alloc(sizeof(float2) * spec * P.nch * P.ngrp);
     } else {
         P.acc.alloc(sizeof(float2) * P.H * std::max(P.nch, P.group * P.nch));
         P.comp.alloc(sizeof(float2) * P.H * P.nch);
@@ -529,9 +535,10 @@ void accum_items(NSPlan& P, int i0, int nz, bool analysis_masks, float2* acc, fl
         }
     }
     if (n > kAccMaxLine) throw ArgError("axis 3 is too long for the accumulating pass of this library");
-    const bool big = f3->mix.R[0] > 20;
-    MixArgs a = mix_args(*f3, P.h1 * P.dims[1], true, false, 2 * sizeof(float2) * (n + 1));
-    const size_t smem = mix_smem_bytes(a.sc, a.lg, a.pitch, false) + 2 * sizeof(float2) * ((size_t)a.pitch << a.lg);
+    const bool big = mix_big(f3->mix);
+    const MixArgs a = mix_args(*f3);
+    const int lg = mix_lines_lg(a, false, 2 * sizeof(float2) * (n + 1)), nlines = P.h1 * P.dims[1];
+    const size_t smem = mix_smem_bytes(a.sc, lg, a.pitch, false) + 2 * sizeof(float2) * ((size_t)a.pitch << lg);
     auto kern = big ? ns_accum_mix_kernel<true> : ns_accum_mix_kernel<false>;
     static bool configured[2] = {false, false};
     if (!configured[big]) {
@@ -540,8 +547,8 @@ void accum_items(NSPlan& P, int i0, int nz, bool analysis_masks, float2* acc, fl
         configured[big] = true;
     }
     int tok = prof_begin("ns_accum_axis3", st);
-    kern<<<(a.nlines + (1 << a.lg) - 1) >> a.lg, mix_threads(a), smem, st>>>(
-        W, P.H, nz, P.tb, P.items.as<NSItem>(), i0, analysis_masks ? 0 : 1, acc, comp, init ? 1 : 0, a);
+    kern<<<(nlines + (1 << lg) - 1) >> lg, mix_threads(a, lg), smem, st>>>(
+        W, P.H, nz, P.tb, P.items.as<NSItem>(), i0, analysis_masks ? 0 : 1, acc, comp, init ? 1 : 0, a, nlines, lg);
     prof_end(tok, st);
     cuda_check(cudaGetLastError(), "ns_accum_mix_kernel launch");
 }
@@ -647,8 +654,13 @@ void ns_analyze_range(NSPlan& P, const float2* X, float* vol, ZMap vz, int es, i
 }
 
 void ns_acc_clear(NSPlan& P, float2* acc, float2* comp, cudaStream_t st) {
+    if (P.slab) return ns_slab_acc_clear(P, acc, comp, st);
     cuda_check(cudaMemsetAsync(acc, 0, sizeof(float2) * ns_spec_elems(P), st), "cudaMemsetAsync(acc)");
     cuda_check(cudaMemsetAsync(comp, 0, sizeof(float2) * ns_spec_elems(P), st), "cudaMemsetAsync(comp)");
+}
+
+float2* ns_range_comp(NSPlan& P, int ch) {
+    return (P.ngrp > 1 ? P.rcomp : P.comp).as<float2>() + ch * ns_spec_elems(P);
 }
 
 float2* ns_comp_grid(NSPlan& P, int ch) { return P.comp.as<float2>() + ch * ns_spec_elems(P); }

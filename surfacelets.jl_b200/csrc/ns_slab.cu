@@ -37,7 +37,7 @@
 #include <cstdlib>
 #include <cstring>
 
-#include "ns_mask.cuh"
+#include "ns_axis3.cuh"
 #include "plan.h"
 #include "prof.h"
 #include "regpass.cuh"
@@ -48,49 +48,6 @@ namespace sfl {
 namespace {
 
 // ── lines along axis 3 of a padded spectrum, restricted to a box ───────────
-
-// Line l = (k1, j) with k1 fastest; column j maps to k2 = j for j <= b2 and
-// to the negative frequencies n2 - (nk2 - j) above.
-struct BoxMap {
-    int nk1, nk2, b2, n2;
-    __device__ __forceinline__ void k12(int l, int& k1, int& k2) const {
-        const int j = l / nk1;
-        k1 = l - j * nk1;
-        k2 = j <= b2 ? j : j + (n2 - nk2);
-    }
-};
-
-// The mask context of a chunk's item on the line (k1, k2): NSMaskLine from the
-// launch's own copy of the item.
-__device__ __forceinline__ NSMaskLine chunk_mask_line(const NSMaskTables& tb, const ChunkSeg& sg, const ChunkItem& it,
-                                                      int k1, int k2, bool synth) {
-    NSMaskLine c;
-    c.low = sg.low;
-    c.plain = 0;
-    c.m = nullptr;
-    c.wa = c.wb = nullptr;
-    c.was = c.wbs = 0;
-    c.lowc = 0.f;
-    c.lowv = nullptr;
-    if (c.low) {
-        c.lowc = tb.vec[tb.low_off[0] + k1] * tb.vec[tb.low_off[1] + k2];
-        c.lowv = tb.vec + tb.low_off[2];
-        return c;
-    }
-    const int l = k1 + tb.h1 * k2;
-    if (synth && !tb.tight) {
-        c.plain = 1;
-        c.m = tb.Bl + (long long)sg.lv * tb.H + l;
-        return c;
-    }
-    c.m = tb.G + (long long)sg.g * tb.H + l;
-    // a plane over (lo, hi): index off + k_lo + dlo * k_hi; axis 3 can only be hi
-    c.wa = tb.planes + it.wa_off + (it.wa_lo == 0 ? k1 : k2) + (it.wa_hi == 2 ? 0 : it.wa_dlo * k2);
-    c.was = it.wa_hi == 2 ? it.wa_dlo : 0;
-    c.wb = tb.planes + it.wb_off + (it.wb_lo == 0 ? k1 : k2) + (it.wb_hi == 2 ? 0 : it.wb_dlo * k2);
-    c.wbs = it.wb_hi == 2 ? it.wb_dlo : 0;
-    return c;
-}
 
 struct L3LoadC {
     const float2* src;
@@ -107,6 +64,50 @@ struct L3LoadC {
     }
     __device__ __forceinline__ float2 get(const Ctx& c, int i) const { return c.p[i * s3]; }
 };
+
+// The sum of the plan's accumulators and their compensations (Kahan steps in
+// the accumulators' order, as merge_groups_kernel's on a cleared spectrum).
+struct L3LoadSum {
+    const float2* acc;
+    const float2* comp;
+    long long zstride, gstride;
+    int ng, P1, s3;
+    BoxMap bx;
+    struct Ctx {
+        const float2* s;
+        const float2* c;
+    };
+    __device__ __forceinline__ Ctx line(int z, int l, bool valid) const {
+        int k1 = 0, k2 = 0;
+        if (valid) bx.k12(l, k1, k2);
+        const long long o = z * zstride + k1 + P1 * k2;
+        return Ctx{acc + o, comp + o};
+    }
+    __device__ __forceinline__ float2 get(const Ctx& c, int i) const {
+        float2 s = make_float2(0.f, 0.f), e = s;
+        for (int g = 0; g < ng; ++g) {
+            const float2 r = c.c[g * gstride + i * s3];
+            kahan_add(s, e, c.s[g * gstride + i * s3]);
+            kahan_add(s, e, make_float2(-r.x, -r.y));
+        }
+        return s;
+    }
+};
+
+// A channel's accumulators added into a caller's spectrum and its compensation.
+__global__ void merge_groups_kernel(const float2* __restrict__ acc, const float2* __restrict__ comp, long long gstride,
+                                    int ng, float2* A, float2* C, long long n) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        float2 s = A[i], e = C[i];
+        for (int g = 0; g < ng; ++g) {
+            const float2 r = comp[g * gstride + i];
+            kahan_add(s, e, acc[g * gstride + i]);
+            kahan_add(s, e, make_float2(-r.x, -r.y));
+        }
+        A[i] = s;
+        C[i] = e;
+    }
+}
 
 struct L3StoreC {
     static constexpr bool kStaged = false;
@@ -140,14 +141,6 @@ constexpr size_t accum_smem() {
     return RegGeom<N>::SMEM + (accum_sums_shared<N>() ? sizeof(float2) * RegGeom<N>::M * RegGeom<N>::N2 * 256 : 0);
 }
 
-// The CTAs of the analysis line pass: tile t takes the line blocks of its
-// segment's box, CTAs [first[t], first[t + 1]), for cnt items from k0.
-struct MaskTiles {
-    int n;
-    int first[kChunkItems + 1];
-    signed char seg[kChunkItems], k0[kChunkItems], cnt[kChunkItems];
-};
-
 // Analysis line pass over up to 8 subbands of one mask group per CTA: a line's
 // X times the group factor is loaded once, then per subband scaled by its
 // wedge planes, transformed along axis 3 and stored.  The tiles of all the
@@ -172,8 +165,7 @@ __global__ void __launch_bounds__(256, mask_minb<N>())
     extern __shared__ float2 xch[];
     X += blockIdx.y * xchs;   // channel
     Y += blockIdx.y * ychs;
-    int t = 0;
-    while (t + 1 < tl.n && (int)blockIdx.x >= tl.first[t + 1]) ++t;
+    const int t = mask_tile_of(tl, blockIdx.x);
     const ChunkSeg& sg = ck.seg[tl.seg[t]];
     const int tid = threadIdx.x;
     const int lp = tid % LP, p = tid / LP;
@@ -250,7 +242,8 @@ __global__ void __launch_bounds__(256, mask_minb<N>())
 // groups of the whole synthesis is compensated
 // (src/transforms/ns_surfacelet.jl:292, 355, 383 accumulate every subband into
 // one spectrum).  CTAs take line blocks of the union box (un) and skip the
-// segments whose box none of their lines meets.
+// segments whose box none of their lines meets.  With several accumulators
+// (P.ngrp, blockIdx.z) mask group g goes to accumulator g mod ngrp.
 //
 // A wedge plane constant along axis 3 commutes with the axis-3 FFT, so the
 // items that share plane b (and the group factor) are combined first,
@@ -261,13 +254,14 @@ template <int N>
 __global__ void __launch_bounds__(256, accum_minb<N>())
     ns_slab_accum_kernel(const float2* __restrict__ Y, long long ystride, int P1, int s3, BoxMap un,
                          const __grid_constant__ NSMaskTables tb, const __grid_constant__ Chunk ck, int synth,
-                         float2* acc, float2* comp, const float2* __restrict__ tw, long long ychs, long long achs) {
+                         float2* acc, float2* comp, const float2* __restrict__ tw, long long ychs, long long achs,
+                         long long agrp) {
     using Ge = RegGeom<N>;
     constexpr int N1 = Ge::N1, N2 = Ge::N2, LP = Ge::LP, E = Ge::M * Ge::N2;
     extern __shared__ float2 xch[];
     Y += blockIdx.y * ychs;   // channel
-    acc += blockIdx.y * achs;
-    comp += blockIdx.y * achs;
+    acc += blockIdx.y * achs + blockIdx.z * agrp;
+    comp += blockIdx.y * achs + blockIdx.z * agrp;
     const int tid = threadIdx.x;
     const int lp = tid % LP, p = tid / LP;
     const int l = blockIdx.x * LP + lp;
@@ -292,6 +286,7 @@ __global__ void __launch_bounds__(256, accum_minb<N>())
 #pragma unroll 1
     for (int sgi = 0; sgi < ck.nseg; ++sgi) {
         const ChunkSeg& sg = ck.seg[sgi];
+        if (sg.ord % (int)gridDim.z != (int)blockIdx.z) continue;   // another accumulator's
         const bool valid = inl && k1 < sg.nk1 && (k2 <= sg.b2 || k2 >= tb.n2 - sg.b2);
         // (the barrier also keeps the previous segment's exchange reads ahead of this one's writes)
         if (ck.nseg > 1 && !__syncthreads_or(valid)) continue;
@@ -481,6 +476,7 @@ Chunk make_chunk(const NSPlan& P, int i0, int nz, bool synth_masks) {
         sg.nz = (short)(e - a);
         sg.nbq = (short)chunk_nbq(P, a, e - a, synth_masks);
         sg.low = f.kind == 1;
+        sg.ord = (short)(f.kind == 1 ? (int)P.boxes.size() - 1 : f.g);
         sg.nk1 = (short)b.nk1;
         sg.nk2 = (short)b.nk2;
         sg.b2 = (short)b.b2;
@@ -562,10 +558,19 @@ void set_volumes(SlabArgs& a, const float* vol, ZMap vz, int es) {
     a.es = es;
 }
 
+// Accumulators of a spectrum acc: the plan's own are P.ngrp (mask group g adds
+// into number g mod ngrp, nch SP apart), a caller's is one.
+int acc_groups(const NSPlan& P, const float2* acc) {
+    const float2* a = P.acc.as<float2>();
+    return acc >= a && acc < a + P.nch * P.SP ? P.ngrp : 1;
+}
+
 // KIND: 0 the forward slab pass, 1 the inverse, 2 the denoiser's shrink pass.
 template <int KIND>
 void launch_slab(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char* tag) {
     const int na = P.dims[0], nb = P.dims[1];
+    if (P.mixed)
+        return (KIND == 0 ? launch_mix_slab_fwd : KIND == 1 ? launch_mix_slab_inv : launch_mix_slab_shrink)(P, a, st, tag);
     if (slab_cluster_supported(na, nb)) {
         if (!launch_slab_cluster(KIND, na, nb, a, P.sms, st, tag)) throw ArgError("no slab kernel for this size");
         return;
@@ -591,11 +596,11 @@ void launch_slab_accum(const NSPlan& P, const Chunk& ck, int synth, float2* acc,
         configured = true;
     }
     const NSBox un = union_box(ck);
-    dim3 grid((un.nk1 * un.nk2 + Ge::LP - 1) / Ge::LP, nch);
+    dim3 grid((un.nk1 * un.nk2 + Ge::LP - 1) / Ge::LP, nch, acc_groups(P, acc));
     int tok = prof_begin("ns_slab_accum_axis3", st);
     ns_slab_accum_kernel<N><<<grid, Ge::THREADS, accum_smem<N>(), st>>>(
         P.work.as<float2>(), P.SP, P.P1, P.P1 * P.dims[1], box_map(P, un), P.tb, ck, synth, acc, comp,
-        P.ffts.at(P.dims[2])->sh.tw, ychs, P.SP);
+        P.ffts.at(P.dims[2])->sh.tw, ychs, P.SP, (long long)P.nch * P.SP);
     prof_end(tok, st);
     cuda_check(cudaGetLastError(), "ns_slab_accum_kernel launch");
 }
@@ -646,6 +651,15 @@ int mask_tiles(const Chunk& ck, int lp, int ipc, MaskTiles& t) {
     return first;
 }
 
+int choose_mask_tiles(const NSPlan& P, const Chunk& ck, int lp, int nch, MaskTiles& tl) {
+    const int cap = mask_ipc_cap(P);
+    int ipc = cap > 0 ? cap : 8;
+    int ctas = mask_tiles(ck, lp, ipc, tl);
+    if (cap == 0 && !t_concurrent)
+        while (ipc > 1 && ctas * nch < P.sms) ctas = mask_tiles(ck, lp, ipc /= 2, tl);
+    return ctas;
+}
+
 template <int N>
 void launch_mask_group(const NSPlan& P, const float2* X, const Chunk& ck, int synth, int nch, long long xchs,
                        long long ychs, cudaStream_t st) {
@@ -658,11 +672,7 @@ void launch_mask_group(const NSPlan& P, const float2* X, const Chunk& ck, int sy
         configured = true;
     }
     MaskTiles tl;
-    const int cap = mask_ipc_cap(P);
-    int ipc = cap > 0 ? cap : 8;
-    int ctas = mask_tiles(ck, Ge::LP, ipc, tl);
-    if (cap == 0 && !t_concurrent)
-        while (ipc > 1 && ctas * nch < P.sms) ctas = mask_tiles(ck, Ge::LP, ipc /= 2, tl);
+    const int ctas = choose_mask_tiles(P, ck, Ge::LP, nch, tl);
     int tok = prof_begin("ns_slab_mask_axis3", st);
     ns_slab_mask_group_kernel<N><<<dim3(ctas, nch), Ge::THREADS, Ge::SMEM, st>>>(
         X, P.P1, P.P1 * P.dims[1], P.tb, ck, tl, synth, P.work.as<float2>(), P.SP, P.ffts.at(P.dims[2])->sh.tw, xchs,
@@ -701,8 +711,15 @@ void slab_irfft3(NSPlan& P, float2* A, float* x, int es, int nch, cudaStream_t s
     prof_bytes("ns_slab_c2r", nch * (box_bytes(P, full) + 4.0 * P.N));
     const BoxMap bx = box_map(P, full);
     const int s3 = P.P1 * P.dims[1];
-    line3<true>(P, L3LoadC{A, P.SP, P.P1, s3, bx}, L3StoreC{A, P.SP, P.P1, s3, bx}, full.nk1 * full.nk2, nch, st,
-                "ns_slab_line3");
+    const int ng = acc_groups(P, A), nl = full.nk1 * full.nk2;
+    const L3StoreC so{A, P.SP, P.P1, s3, bx};
+    if (ng > 1) {
+        const long long ch0 = A - P.acc.as<float2>();
+        line3<true>(P, L3LoadSum{A, P.comp.as<float2>() + ch0, P.SP, (long long)P.nch * P.SP, ng, P.P1, s3, bx}, so, nl,
+                    nch, st, "ns_slab_line3");
+    } else {
+        line3<true>(P, L3LoadC{A, P.SP, P.P1, s3, bx}, so, nl, nch, st, "ns_slab_line3");
+    }
     SlabArgs a = slab_args(P, full_chunk(P), nch);
     a.spec_chstride = P.SP;
     a.spec = A;
@@ -717,6 +734,14 @@ void slab_mask_pass(NSPlan& P, const float2* X, const Chunk& ck, bool synth_mask
     prof_bytes("ns_slab_mask_axis3", nch * (1.5 * segs_bytes(P, ck) + items_bytes(P, ck)));
     const int sy = synth_masks ? 1 : 0;
     const long long xc = P.SP, yc = ych_stride(P);
+    if (P.mixed) {
+        MaskTiles tl;
+        choose_mask_tiles(P, ck, mix_axis3_lines(P), nch, tl);
+        int tok = prof_begin("ns_slab_mask_axis3", st);
+        launch_mix_mask(P, X, ck, tl, sy, P.work.as<float2>(), nch, xc, yc, st);
+        prof_end(tok, st);
+        return;
+    }
     switch (P.dims[2]) {
         case 16: launch_mask_group<16>(P, X, ck, sy, nch, xc, yc, st); return;
         case 32: launch_mask_group<32>(P, X, ck, sy, nch, xc, yc, st); return;
@@ -737,6 +762,13 @@ void slab_accum_pass(NSPlan& P, const Chunk& ck, bool analysis_masks, float2* ac
     prof_bytes("ns_slab_accum_axis3", nch * (items_bytes(P, ck) + 4.5 * segs_bytes(P, ck)));
     const int sy = analysis_masks ? 0 : 1;
     const long long yc = ych_stride(P);
+    if (P.mixed) {
+        int tok = prof_begin("ns_slab_accum_axis3", st);
+        launch_mix_accum(P, ck, box_map(P, union_box(ck)), sy, P.work.as<float2>(), acc, comp, nch, acc_groups(P, acc),
+                         yc, st);
+        prof_end(tok, st);
+        return;
+    }
     switch (P.dims[2]) {
         case 16: launch_slab_accum<16>(P, ck, sy, acc, comp, nch, yc, st); return;
         case 32: launch_slab_accum<32>(P, ck, sy, acc, comp, nch, yc, st); return;
@@ -860,11 +892,45 @@ NSBox ns_make_box(int nk1, int b2, int n2) {
     return b;
 }
 
+void ns_slab_acc_clear(NSPlan& P, float2* acc, float2* comp, cudaStream_t st) {
+    const int ng = acc_groups(P, acc);
+    for (int g = 0; g < ng; ++g) {
+        const long long o = (long long)g * P.nch * P.SP;
+        cuda_check(cudaMemsetAsync(acc + o, 0, sizeof(float2) * P.SP, st), "cudaMemsetAsync(acc)");
+        cuda_check(cudaMemsetAsync(comp + o, 0, sizeof(float2) * P.SP, st), "cudaMemsetAsync(comp)");
+    }
+}
+
+void ns_merge_groups(NSPlan& P, int ch, float2* A, float2* C, cudaStream_t st) {
+    const long long blocks = std::min<long long>((P.SP + 255) / 256, 8LL * P.sms);
+    merge_groups_kernel<<<(unsigned)blocks, 256, 0, st>>>(P.acc.as<float2>() + ch * P.SP, P.comp.as<float2>() + ch * P.SP,
+                                                          (long long)P.nch * P.SP, P.ngrp, A, C, P.SP);
+    cuda_check(cudaGetLastError(), "merge_groups_kernel launch");
+}
+
+// Accumulators of the synthesis.  A CTA of the axis-3 pass walks the terms of
+// its lines one after the other, and a small spectrum has too few lines to
+// fill the GPU (66 CTAs at 64^3, 13 us a term): its mask groups then go to
+// several accumulators, summed by the inverse FFT's first pass.
+int ns_slab_groups(const NSPlan& P) {
+    const long long lines = (long long)P.h1 * P.dims[1];
+    return lines <= 5000 ? 4 : (lines <= 10000 ? 2 : 1);
+}
+
+void ns_use_mixed(NSPlan& P) {
+    if (!ns_mix_slab_supported(P))
+        throw ArgError("the mixed-radix slab pipeline does not support size " + std::to_string(P.dims[0]) + "x" +
+                       std::to_string(P.dims[1]) + "x" + std::to_string(P.dims[2]));
+    P.slab = P.mixed = true;
+    ns_alloc_scratch(P);
+}
+
 void ns_use_slabs(NSPlan& P) {
     if (!ns_slab_supported(P.dims[0], P.dims[1], P.dims[2]))
         throw ArgError("the slab pipeline does not support size " + std::to_string(P.dims[0]) + "x" +
                        std::to_string(P.dims[1]) + "x" + std::to_string(P.dims[2]));
     P.slab = true;
+    P.mixed = false;
     ns_alloc_scratch(P);
 }
 
@@ -888,8 +954,8 @@ void ns_slab_synthesize(NSPlan& P, const void* c, void* x, cudaStream_t st, bool
     const int nch = P.nch;
     float2* A = P.acc.as<float2>();
     float2* K = P.comp.as<float2>();
-    cuda_check(cudaMemsetAsync(A, 0, sizeof(float2) * P.SP * nch, st), "cudaMemsetAsync(acc)");
-    cuda_check(cudaMemsetAsync(K, 0, sizeof(float2) * P.SP * nch, st), "cudaMemsetAsync(comp)");
+    cuda_check(cudaMemsetAsync(A, 0, sizeof(float2) * P.SP * nch * P.ngrp, st), "cudaMemsetAsync(acc)");
+    cuda_check(cudaMemsetAsync(K, 0, sizeof(float2) * P.SP * nch * P.ngrp, st), "cudaMemsetAsync(comp)");
     for (int i0 = 0, i1; i0 < P.S; i0 = i1) {
         i1 = chunk_end(P, i0);
         slab_synth_items(P, static_cast<const float*>(c), ns_subband_map(P, i0, nch), nch, i0, i1 - i0,

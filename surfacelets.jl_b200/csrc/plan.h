@@ -138,6 +138,8 @@ struct NSPlan {
     HostWord status;        // status word of bounded waits (0 = fine), written by the kernels
     // slab pipeline (spectra with the axis-1 pitch padded to P1)
     bool slab = false;
+    bool mixed = false;             // the slab pipeline on the mixed-radix FFT (any lengths)
+    int ngrp = 1;                   // accumulators of the synthesis (ns_slab_groups)
     int P1 = 0;
     long long SP = 0;               // P1 * n2 * n3
     std::vector<NSBox> boxes;       // per mask group, then the lowpass
@@ -146,7 +148,8 @@ struct NSPlan {
     std::map<int, std::unique_ptr<FFTLen>> ffts;
     DevMem X;        // nch spectra
     DevMem work;     // group spectra
-    DevMem acc, comp;   // nch accumulators (+ Kahan compensation)
+    DevMem acc, comp;   // ngrp nch accumulators (+ Kahan compensation)
+    DevMem rcomp;       // compensation of a caller's spectrum (item ranges), with several accumulators
     DevMem band, maxbits;   // float32 subbands of a chunk and their peaks (bfloat16 coefficients)
     // streaming state
     int stream_mode = 0;    // 0 idle, 1 analyzing, 2 synthesizing
@@ -192,6 +195,13 @@ bool ns_slab_supported(int n1, int n2, int n3);
 // larger CTAs over filling the GPU alone.
 void ns_set_concurrent(bool on);
 void ns_use_slabs(NSPlan& P);
+bool ns_mix_slab_supported(const NSPlan& P);
+void ns_use_mixed(NSPlan& P);
+int ns_slab_groups(const NSPlan& P);
+void ns_slab_acc_clear(NSPlan& P, float2* acc, float2* comp, cudaStream_t st);
+// The plan's accumulators of channel ch added into a caller's spectrum A with compensation C.
+void ns_merge_groups(NSPlan& P, int ch, float2* A, float2* C, cudaStream_t st);
+float2* ns_range_comp(NSPlan& P, int ch);
 int ns_slab_slots(const NSPlan& P);
 NSBox ns_make_box(int nk1, int b2, int n2);
 NSBox ns_table_box(const std::vector<double>& g, int h1, int n2, int n3);

@@ -35,7 +35,7 @@ struct ChunkSeg {
     short nbq;                    // > 0: nbq plane-b wedges times whole rows of plane-a wedges constant along axis 3
     short low;                    // the lowpass
     short nk1, nk2, b2;           // support box
-    short pad;
+    short ord;                    // mask group of the plan, the lowpass last: the accumulator is ord mod their number
 };
 struct Chunk {
     int nz, nseg;

@@ -423,7 +423,7 @@ class Workspace:
     def set_group(self, group):
         check(lib.sfl_plan_set_group(self._h, int(group)))
 
-    PIPELINES = {"lines": 0, "planes": 1, "slabs": 2}
+    PIPELINES = {"lines": 0, "planes": 1, "slabs": 2, "mixed": 3}
 
     def tuning(self):
         """(pipeline name, group) in use."""
@@ -455,8 +455,9 @@ class Workspace:
 
     def set_pipeline(self, name):
         """NSSurfacelet kernel pipeline: "slabs" (the default where the size
-        allows) or "lines" ("planes", the retired plane-major pipeline, is
-        refused by the library)."""
+        allows), "mixed" (the same passes for any lengths whose slabs fit
+        shared memory, the default there) or "lines" ("planes", the retired
+        plane-major pipeline, is refused by the library)."""
         if name not in self.PIPELINES:
             raise ArgumentError(f"unknown pipeline {name!r}; expected one of {sorted(self.PIPELINES)}")
         check(lib.sfl_plan_set_pipeline(self._h, self.PIPELINES[name]))

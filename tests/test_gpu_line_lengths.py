@@ -1,6 +1,7 @@
-"""The mixed-radix line pass at the lengths where its schedule changes: one,
+"""The mixed-radix line FFT at the lengths where its schedule changes: one,
 two and three radices, the largest radices, large primes (alone, with a small
-factor, two of them), along each axis, against the float64 oracle.
+factor, two of them), along each axis, on the line passes and on the slab
+passes built from it, against the float64 oracle.
 
 Tolerance: float32 rounding u = 6e-8 grows as sqrt(terms) along a sum of a
 large prime's q / 2 products and as sqrt(log2 n) along the other steps; a
@@ -21,12 +22,16 @@ LENGTHS = [2, 7, 17, 19, 20, 23, 29, 34, 45, 46, 77, 91, 100, 109, 125, 150, 200
 @pytest.mark.gpu
 @pytest.mark.parametrize("axis", [0, 1, 2])
 @pytest.mark.parametrize("n", LENGTHS)
-def test_line_lengths_match_oracle(sfl, n, axis):
+@pytest.mark.parametrize("pipeline", ["lines", "mixed"])
+def test_line_lengths_match_oracle(sfl, n, axis, pipeline):
     dims = [6, 5, 8]
     dims[axis] = n
     dims = tuple(dims)
     x = np.random.default_rng(n).standard_normal(dims).astype(np.float32)
     ws = sfl.make_workspace(sfl.HourglassFB(bernstein_order=6), "float32", dims)
+    if pipeline == "mixed" and n >= 1000:
+        pytest.skip("tiles of this length leave no room for a slab")
+    ws.set_pipeline(pipeline)
     bands = sfl.hourglass_decompose(ws, sfl.to_device(x))
     ref = N.hourglass_decompose(x, dims, 6, 1)
     for b, r in zip(bands, ref):
