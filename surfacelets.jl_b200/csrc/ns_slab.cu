@@ -65,45 +65,51 @@ struct L3LoadC {
     __device__ __forceinline__ float2 get(const Ctx& c, int i) const { return c.p[i * s3]; }
 };
 
-// The sum of the plan's accumulators and their compensations (Kahan steps in
-// the accumulators' order, as merge_groups_kernel's on a cleared spectrum).
-struct L3LoadSum {
+// The plan's NG accumulators less their compensations, summed in the
+// accumulators' order.
+template <int NG>
+struct GroupSum {
     const float2* acc;
     const float2* comp;
-    long long zstride, gstride;
-    int ng, P1, s3;
+    long long gstride;
+    __device__ __forceinline__ float2 at(long long o) const {
+        float2 s[NG], e[NG];
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+            s[g] = __ldg(acc + g * gstride + o);
+            e[g] = __ldg(comp + g * gstride + o);
+        }
+        float2 v = c_sub(s[0], e[0]);
+#pragma unroll
+        for (int g = 1; g < NG; ++g) v = c_add(v, c_sub(s[g], e[g]));
+        return v;
+    }
+};
+
+template <int NG>
+struct L3LoadSum {
+    GroupSum<NG> gs;
+    long long zstride;
+    int P1, s3;
     BoxMap bx;
     struct Ctx {
-        const float2* s;
-        const float2* c;
+        long long o;
     };
     __device__ __forceinline__ Ctx line(int z, int l, bool valid) const {
         int k1 = 0, k2 = 0;
         if (valid) bx.k12(l, k1, k2);
-        const long long o = z * zstride + k1 + P1 * k2;
-        return Ctx{acc + o, comp + o};
+        return Ctx{z * zstride + k1 + P1 * k2};
     }
-    __device__ __forceinline__ float2 get(const Ctx& c, int i) const {
-        float2 s = make_float2(0.f, 0.f), e = s;
-        for (int g = 0; g < ng; ++g) {
-            const float2 r = c.c[g * gstride + i * s3];
-            kahan_add(s, e, c.s[g * gstride + i * s3]);
-            kahan_add(s, e, make_float2(-r.x, -r.y));
-        }
-        return s;
-    }
+    __device__ __forceinline__ float2 get(const Ctx& c, int i) const { return gs.at(c.o + i * s3); }
 };
 
-// A channel's accumulators added into a caller's spectrum and its compensation.
-__global__ void merge_groups_kernel(const float2* __restrict__ acc, const float2* __restrict__ comp, long long gstride,
-                                    int ng, float2* A, float2* C, long long n) {
+// A channel's accumulators added into a caller's spectrum and its compensation
+// (on a cleared one, GroupSum's values exactly).
+template <int NG>
+__global__ void merge_groups_kernel(GroupSum<NG> gs, float2* A, float2* C, long long n) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         float2 s = A[i], e = C[i];
-        for (int g = 0; g < ng; ++g) {
-            const float2 r = comp[g * gstride + i];
-            kahan_add(s, e, acc[g * gstride + i]);
-            kahan_add(s, e, make_float2(-r.x, -r.y));
-        }
+        kahan_add(s, e, gs.at(i));
         A[i] = s;
         C[i] = e;
     }
@@ -713,13 +719,14 @@ void slab_irfft3(NSPlan& P, float2* A, float* x, int es, int nch, cudaStream_t s
     const int s3 = P.P1 * P.dims[1];
     const int ng = acc_groups(P, A), nl = full.nk1 * full.nk2;
     const L3StoreC so{A, P.SP, P.P1, s3, bx};
-    if (ng > 1) {
-        const long long ch0 = A - P.acc.as<float2>();
-        line3<true>(P, L3LoadSum{A, P.comp.as<float2>() + ch0, P.SP, (long long)P.nch * P.SP, ng, P.P1, s3, bx}, so, nl,
-                    nch, st, "ns_slab_line3");
-    } else {
+    const float2* K = P.comp.as<float2>() + (ng > 1 ? A - P.acc.as<float2>() : 0);
+    const long long gs = (long long)P.nch * P.SP;
+    if (ng == 4)
+        line3<true>(P, L3LoadSum<4>{{A, K, gs}, P.SP, P.P1, s3, bx}, so, nl, nch, st, "ns_slab_line3");
+    else if (ng == 2)
+        line3<true>(P, L3LoadSum<2>{{A, K, gs}, P.SP, P.P1, s3, bx}, so, nl, nch, st, "ns_slab_line3");
+    else
         line3<true>(P, L3LoadC{A, P.SP, P.P1, s3, bx}, so, nl, nch, st, "ns_slab_line3");
-    }
     SlabArgs a = slab_args(P, full_chunk(P), nch);
     a.spec_chstride = P.SP;
     a.spec = A;
@@ -903,14 +910,18 @@ void ns_slab_acc_clear(NSPlan& P, float2* acc, float2* comp, cudaStream_t st) {
 
 void ns_merge_groups(NSPlan& P, int ch, float2* A, float2* C, cudaStream_t st) {
     const long long blocks = std::min<long long>((P.SP + 255) / 256, 8LL * P.sms);
-    merge_groups_kernel<<<(unsigned)blocks, 256, 0, st>>>(P.acc.as<float2>() + ch * P.SP, P.comp.as<float2>() + ch * P.SP,
-                                                          (long long)P.nch * P.SP, P.ngrp, A, C, P.SP);
+    const float2 *a = P.acc.as<float2>() + ch * P.SP, *k = P.comp.as<float2>() + ch * P.SP;
+    const long long gs = (long long)P.nch * P.SP;
+    if (P.ngrp == 4)
+        merge_groups_kernel<4><<<(unsigned)blocks, 256, 0, st>>>(GroupSum<4>{a, k, gs}, A, C, P.SP);
+    else
+        merge_groups_kernel<2><<<(unsigned)blocks, 256, 0, st>>>(GroupSum<2>{a, k, gs}, A, C, P.SP);
     cuda_check(cudaGetLastError(), "merge_groups_kernel launch");
 }
 
 // Accumulators of the synthesis.  A CTA of the axis-3 pass walks the terms of
 // its lines one after the other, and a small spectrum has too few lines to
-// fill the GPU (66 CTAs at 64^3, 13 us a term): its mask groups then go to
+// fill the GPU (66 CTAs at 64^3, 3.5 us a term): its mask groups then go to
 // several accumulators, summed by the inverse FFT's first pass.
 int ns_slab_groups(const NSPlan& P) {
     const long long lines = (long long)P.h1 * P.dims[1];
