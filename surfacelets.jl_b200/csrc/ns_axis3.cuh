@@ -84,6 +84,20 @@ __device__ __forceinline__ int mask_tile_of(const MaskTiles& tl, int cta) {
     return t;
 }
 
+// The axis-3 passes with the length known at compile time (ns_axis3_mask.cu,
+// ns_axis3_accum.cu), and the slab passes of the same lengths
+// (ns_any_slab.cuh).
+bool axis3_len(int n);
+int axis3_lines(int n);   // lines a CTA of the analysis pass takes
+void launch_axis3_mask(const NSPlan& P, const float2* X, const Chunk& ck, const MaskTiles& tl, int synth, float2* Y,
+                       int nch, long long xchs, long long ychs, cudaStream_t st);
+void launch_axis3_accum(const NSPlan& P, const Chunk& ck, const BoxMap& un, int synth, const float2* Y, float2* acc,
+                        float2* comp, int nch, int ngrp, long long ychs, cudaStream_t st);
+bool any_slab_fits(const NSPlan& P);
+void launch_any_slab_fwd(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char* tag);
+void launch_any_slab_inv(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char* tag);
+void launch_any_slab_shrink(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char* tag);
+
 // The passes for any axis lengths (ns_mix_slab.cuh, ns_mix_axis3.cu).
 bool mix_slab_fits(const NSPlan& P);
 void launch_mix_slab_fwd(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char* tag);

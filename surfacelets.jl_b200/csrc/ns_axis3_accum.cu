@@ -1,0 +1,207 @@
+// The synthesis axis-3 pass of the slab pipeline, lengths of SFL_ANY_LENGTHS.
+#include "anyfft.cuh"
+#include "ns_axis3.cuh"
+#include "prof.h"
+
+namespace sfl {
+
+namespace {
+
+// Lengths whose sums go to shared memory (their register form spills).
+template <int N>
+constexpr bool accum_sums_shared() { return AnyLine<N>::E > 8; }
+template <int N>
+constexpr size_t accum_smem() {
+    return AnyGeom<N>::SMEM + (accum_sums_shared<N>() ? sizeof(float2) * AnyLine<N>::E * AnyGeom<N>::THREADS : 0);
+}
+
+// Synthesis line pass over a chunk's segments: per segment FFT_3 of every item
+// times its mask, summed in float32 over the segment's terms, then added into
+// the accumulator with one Kahan step against the compensation grid comp: the
+// compensation carries across segments and launches, so the sum over the mask
+// groups of the whole synthesis is compensated
+// (src/transforms/ns_surfacelet.jl:292, 355, 383 accumulate every subband into
+// one spectrum).  CTAs take line blocks of the union box (un) and skip the
+// segments whose box none of their lines meets.  With several accumulators
+// (P.ngrp, blockIdx.z) mask group g goes to accumulator g mod ngrp.
+//
+// A wedge plane constant along axis 3 commutes with the axis-3 FFT, so the
+// items that share plane b (and the group factor) are combined first,
+// sum_p wa_p(k1, k2) Y_pq, and transformed once: with nbq > 0 the segment is
+// nbq plane-b wedges q times whole rows p (item t = p nbq + q); otherwise
+// every item is its own term.  Terms are added in q order.
+template <int N>
+__global__ void __launch_bounds__(256, 2)
+    ns_slab_accum_kernel(const float2* __restrict__ Y, long long ystride, int P1, int s3, BoxMap un,
+                         const __grid_constant__ NSMaskTables tb, const __grid_constant__ Chunk ck, int synth,
+                         float2* acc, float2* comp, const float2* __restrict__ tw, long long ychs, long long achs,
+                         long long agrp) {
+    using Ge = AnyGeom<N>;
+    constexpr int N1 = Ge::N1, N2 = Ge::N2, LP = Ge::LP, E = Ge::E;
+    extern __shared__ float2 xch[];
+    Y += blockIdx.y * ychs;   // channel
+    acc += blockIdx.y * achs + blockIdx.z * agrp;
+    comp += blockIdx.y * achs + blockIdx.z * agrp;
+    const int tid = threadIdx.x;
+    const int lp = tid % LP, p = tid / LP;
+    const int l = blockIdx.x * LP + lp;
+    const bool inl = l < un.nk1 * un.nk2;
+    int k1 = 0, k2 = 0;
+    if (inl) un.k12(l, k1, k2);
+    float2* xl = xch + lp * Ge::XLINE;
+    // a segment's sums: in registers, or (lengths whose registers would spill) in shared memory after the
+    // exchange rows, value q of thread t at [q * THREADS + t]
+    constexpr bool kSumsShared = accum_sums_shared<N>();
+    float2 sr[kSumsShared ? 1 : E];
+    float2* ss = xch + LP * Ge::XLINE + tid;
+    auto sum = [&](int q) -> float2& {
+        if constexpr (kSumsShared)
+            return ss[q * Ge::THREADS];
+        else
+            return sr[q];
+    };
+    const int si = tb.h1 * tb.n2;
+    const bool wedge_masks = !(synth && !tb.tight);
+    const float2* yl = Y + k1 + P1 * k2;
+#pragma unroll 1
+    for (int sgi = 0; sgi < ck.nseg; ++sgi) {
+        const ChunkSeg& sg = ck.seg[sgi];
+        if (sg.ord % (int)gridDim.z != (int)blockIdx.z) continue;   // another accumulator's
+        const bool valid = inl && k1 < sg.nk1 && (k2 <= sg.b2 || k2 >= tb.n2 - sg.b2);
+        // (the barrier also keeps the previous segment's exchange reads ahead of this one's writes)
+        if (ck.nseg > 1 && !__syncthreads_or(valid)) continue;
+#pragma unroll
+        for (int q = 0; q < E; ++q) sum(q) = make_float2(0.f, 0.f);
+        // the group factor of the line (group table, bandpass table or the lowpass factors), once for all items
+        float gf[E];
+        {
+            const NSMaskLine m0 = chunk_mask_line(tb, sg, ck.item[sg.i0], k1, k2, synth != 0);
+#pragma unroll
+            for (int j = 0; j < Ge::M; ++j)
+#pragma unroll
+                for (int k = 0; k < N2; ++k) {
+                    const int k3 = Ge::has(p, j) ? (p + N2 * j) + N1 * k : 0;
+                    gf[j * N2 + k] = m0.low ? m0.lowc * m0.lowv[k3] : m0.m[(long long)k3 * si];
+                }
+        }
+        const int nbq = sg.nbq;
+        const int rows = nbq > 0 ? sg.nz / nbq : 1;
+        const int nterms = nbq > 0 ? nbq : sg.nz;
+#pragma unroll 1
+        for (int t = 0; t < nterms; ++t) {
+            const ChunkItem& it0 = ck.item[sg.i0 + t];
+            const bool before = wedge_masks && !sg.low && it0.wa_hi != 2;   // plane a applied before the FFT
+            // the term: sum_p wa_p Y_pq (one item with weight 1 when plane a varies along the line; x 1 is
+            // exact).  The loads of the next item are in flight while the current one is added.
+            const int nt = before ? rows : 1;
+            auto weight = [&](int z) {
+                const ChunkItem& it = ck.item[z];
+                return before ? __ldg(tb.planes + it.wa_off + (it.wa_lo == 0 ? k1 : k2) + it.wa_dlo * k2) : 1.f;
+            };
+            float2 v[N1], yb[N1];
+            const int z0 = sg.i0 + t;
+            float wz = weight(z0);
+            {
+                const float2* yz = yl + z0 * ystride;
+#pragma unroll
+                for (int r = 0; r < N1; ++r) yb[r] = valid ? yz[(long long)(p + N2 * r) * s3] : make_float2(0.f, 0.f);
+            }
+#pragma unroll 1
+            for (int pp = 0; pp < nt; ++pp) {
+                const float az = wz;
+                if constexpr (N1 <= 16) {
+                    // a second buffer for the next item's loads (long lines would spill it)
+                    float2 cur[N1];
+#pragma unroll
+                    for (int r = 0; r < N1; ++r) cur[r] = yb[r];
+                    if (pp + 1 < nt) {
+                        const int z = z0 + (pp + 1) * nbq;
+                        const float2* yz = yl + z * ystride;
+                        wz = weight(z);
+#pragma unroll
+                        for (int r = 0; r < N1; ++r)
+                            yb[r] = valid ? yz[(long long)(p + N2 * r) * s3] : make_float2(0.f, 0.f);
+                    }
+#pragma unroll
+                    for (int r = 0; r < N1; ++r) v[r] = pp == 0 ? c_scale(cur[r], az) : c_fma(cur[r], az, v[r]);
+                } else {
+#pragma unroll
+                    for (int r = 0; r < N1; ++r) v[r] = pp == 0 ? c_scale(yb[r], az) : c_fma(yb[r], az, v[r]);
+                    if (pp + 1 < nt) {
+                        const int z = z0 + (pp + 1) * nbq;
+                        const float2* yz = yl + z * ystride;
+                        wz = weight(z);
+#pragma unroll
+                        for (int r = 0; r < N1; ++r)
+                            yb[r] = valid ? yz[(long long)(p + N2 * r) * s3] : make_float2(0.f, 0.f);
+                    }
+                }
+            }
+            float2 u[E];
+            if (t > 0) __syncthreads();   // the exchange rows were read for the previous term
+            any_block_fft<N, false>(v, p, xl, tw, u);
+            // the term's first item carries plane b and the group factor
+            const NSMaskLine mk = chunk_mask_line(tb, sg, it0, k1, k2, synth != 0);
+            const bool wedges = !(mk.low || mk.plain);
+#pragma unroll
+            for (int j = 0; j < Ge::M; ++j)
+#pragma unroll
+                for (int k = 0; k < N2; ++k) {
+                    const int k3 = Ge::has(p, j) ? (p + N2 * j) + N1 * k : 0;
+                    const float g = gf[j * N2 + k];
+                    const float m = !wedges ? g : (before ? g * mk.wb[k3 * mk.wbs] : g * (mk.wa[k3 * mk.was] * mk.wb[k3 * mk.wbs]));
+                    float2& tsum = sum(j * N2 + k);
+                    tsum = make_float2(fmaf(u[j * N2 + k].x, m, tsum.x), fmaf(u[j * N2 + k].y, m, tsum.y));
+                }
+        }
+        if (valid) {
+            float2* a = acc + k1 + P1 * k2;
+            float2* ca = comp + k1 + P1 * k2;
+#pragma unroll
+            for (int j = 0; j < Ge::M; ++j)
+                if (Ge::has(p, j)) {
+#pragma unroll
+                    for (int k = 0; k < N2; ++k) {
+                        const int o = ((p + N2 * j) + N1 * k) * s3;
+                        float2 sv = a[o], cv = ca[o];
+                        kahan_add(sv, cv, sum(j * N2 + k));
+                        a[o] = sv;
+                        ca[o] = cv;
+                    }
+                }
+        }
+    }
+}
+
+template <int N>
+void launch_n(const NSPlan& P, const Chunk& ck, const BoxMap& un, int synth, const float2* Y, float2* acc, float2* comp,
+              int nch, int ngrp, long long ychs, cudaStream_t st) {
+    using Ge = AnyGeom<N>;
+    static bool configured = false;
+    if (!configured) {
+        cuda_check(cudaFuncSetAttribute(ns_slab_accum_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)accum_smem<N>()),
+                   "cudaFuncSetAttribute");
+        configured = true;
+    }
+    const dim3 grid((un.nk1 * un.nk2 + Ge::LP - 1) / Ge::LP, nch, ngrp);
+    ns_slab_accum_kernel<N><<<grid, Ge::THREADS, accum_smem<N>(), st>>>(
+        Y, P.SP, P.P1, P.P1 * P.dims[1], un, P.tb, ck, synth, acc, comp, P.ffts.at(N)->sh.tw, ychs, P.SP,
+        (long long)P.nch * P.SP);
+    cuda_check(cudaGetLastError(), "ns_slab_accum_kernel launch");
+}
+
+}  // namespace
+
+void launch_axis3_accum(const NSPlan& P, const Chunk& ck, const BoxMap& un, int synth, const float2* Y, float2* acc,
+                        float2* comp, int nch, int ngrp, long long ychs, cudaStream_t st) {
+    switch (P.dims[2]) {
+#define SFL_AXIS3_CASE(N_) \
+    case N_: launch_n<N_>(P, ck, un, synth, Y, acc, comp, nch, ngrp, ychs, st); return;
+        SFL_ANY_LENGTHS(SFL_AXIS3_CASE)
+#undef SFL_AXIS3_CASE
+    }
+    throw ArgError("no axis-3 pass of this length");
+}
+
+}  // namespace sfl

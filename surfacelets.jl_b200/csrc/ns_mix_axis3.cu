@@ -288,7 +288,7 @@ bool ns_mix_slab_supported(const NSPlan& P) {
     size_t smem;
     mix_axis3(P, smem);
     // 32-bit offsets within a spectrum
-    return mix_slab_fits(P) && smem <= kSlabSmemOneCta && P.SP < (1LL << 31) && P.dims[2] <= 4096;
+    return (any_slab_fits(P) || mix_slab_fits(P)) && smem <= kSlabSmemOneCta && P.SP < (1LL << 31) && P.dims[2] <= 4096;
 }
 
 int mix_axis3_lines(const NSPlan& P) {

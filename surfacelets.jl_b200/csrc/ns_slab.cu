@@ -132,271 +132,6 @@ struct L3StoreC {
     __device__ __forceinline__ void put(const Ctx& c, int k, float2 v) const { c.p[k * s3] = v; }
 };
 
-// Resident CTAs an SM the register budget aims at: two (128 registers a
-// thread) where the line geometry fits, one for the long-N1 lengths 96 and
-// 160 (24 and 40 values a thread) and for 256 in the accumulation.
-template <int N>
-constexpr int mask_minb() { return (N == 96 || N == 160) ? 1 : 2; }
-template <int N>
-constexpr int accum_minb() { return (N == 96 || N == 160 || N >= 256) ? 1 : 2; }
-// Accumulation lengths whose sums go to shared memory (their register form spills).
-template <int N>
-constexpr bool accum_sums_shared() { return N == 96 || N == 128 || N == 160; }
-template <int N>
-constexpr size_t accum_smem() {
-    return RegGeom<N>::SMEM + (accum_sums_shared<N>() ? sizeof(float2) * RegGeom<N>::M * RegGeom<N>::N2 * 256 : 0);
-}
-
-// Analysis line pass over up to 8 subbands of one mask group per CTA: a line's
-// X times the group factor is loaded once, then per subband scaled by its
-// wedge planes, transformed along axis 3 and stored.  The tiles of all the
-// chunk's mask groups share the launch.
-//
-// Wedge planes constant along axis 3 (plane a of hourglasses 1 and 2, over
-// (k1, k2)) are a per-line scalar and commute with the axis-3 FFT, so they
-// are applied after it: Y_s = wa_p(k1, k2) IFFT_3(X G wb_q).  With nbq > 0
-// the segment is nbq plane-b wedges q times whole rows of plane-a wedges p
-// (item t = p nbq + q); the CTA takes the items q-major, and consecutive
-// items of one q share a single FFT.  Every such item uses this order of
-// operations whether or not it shares, so the values do not depend on the
-// chunking.
-template <int N>
-__global__ void __launch_bounds__(256, mask_minb<N>())
-    ns_slab_mask_group_kernel(const float2* __restrict__ X, int P1, int s3, const __grid_constant__ NSMaskTables tb,
-                              const __grid_constant__ Chunk ck, const __grid_constant__ MaskTiles tl, int synth,
-                              float2* Y, long long ystride, const float2* __restrict__ tw, long long xchs,
-                              long long ychs) {
-    using Ge = RegGeom<N>;
-    constexpr int N1 = Ge::N1, N2 = Ge::N2, LP = Ge::LP, E = Ge::M * Ge::N2;
-    extern __shared__ float2 xch[];
-    X += blockIdx.y * xchs;   // channel
-    Y += blockIdx.y * ychs;
-    const int t = mask_tile_of(tl, blockIdx.x);
-    const ChunkSeg& sg = ck.seg[tl.seg[t]];
-    const int tid = threadIdx.x;
-    const int lp = tid % LP, p = tid / LP;
-    const int l = ((int)blockIdx.x - tl.first[t]) * LP + lp;
-    const bool valid = l < sg.nk1 * sg.nk2;
-    int k1 = 0, k2 = 0;
-    if (valid) BoxMap{sg.nk1, sg.nk2, sg.b2, tb.n2}.k12(l, k1, k2);
-    float2* xl = xch + lp * Ge::XLINE;
-    const int k0 = tl.k0[t], kend = k0 + tl.cnt[t];
-    const int nbq = sg.nbq, rows = nbq > 0 ? sg.nz / nbq : 0;
-    auto zof = [&](int k) { return sg.i0 + (nbq > 0 ? (k % rows) * nbq + k / rows : k); };
-    // the group factor of the line (group table, bandpass table or the lowpass factors)
-    float2 xg[N1];
-    {
-        const NSMaskLine m0 = chunk_mask_line(tb, sg, ck.item[sg.i0], k1, k2, synth != 0);
-        const float2* xp = X + k1 + P1 * k2;
-        const int si = tb.h1 * tb.n2;
-#pragma unroll
-        for (int r = 0; r < N1; ++r) {
-            const int i = p + N2 * r;
-            const float g = m0.low ? m0.lowc * m0.lowv[i] : m0.m[(long long)i * si];
-            xg[r] = valid ? c_scale(xp[(long long)i * s3], g) : make_float2(0.f, 0.f);
-        }
-    }
-    float2 u[E];
-#pragma unroll 1
-    for (int k = k0; k < kend; ++k) {
-        const int z = zof(k);
-        const NSMaskLine mk = chunk_mask_line(tb, sg, ck.item[z], k1, k2, synth != 0);
-        const bool wedges = !(mk.low || mk.plain);
-        // plane a constant along the line: applied after the FFT
-        const bool after = wedges && mk.was == 0;
-        const bool reuse = after && nbq > 0 && k > k0 && (k - 1) / rows == k / rows;   // same q: uniform
-        if (!reuse) {
-            float2 v[N1];
-            if (!wedges) {
-#pragma unroll
-                for (int r = 0; r < N1; ++r) v[r] = xg[r];
-            } else if (after) {
-#pragma unroll
-                for (int r = 0; r < N1; ++r) v[r] = c_scale(xg[r], mk.wb[(p + N2 * r) * mk.wbs]);
-            } else if (mk.wbs == 0) {
-                const float b0 = mk.wb[0];
-#pragma unroll
-                for (int r = 0; r < N1; ++r) v[r] = c_scale(xg[r], mk.wa[(p + N2 * r) * mk.was] * b0);
-            } else {
-#pragma unroll
-                for (int r = 0; r < N1; ++r) {
-                    const int i = p + N2 * r;
-                    v[r] = c_scale(xg[r], mk.wa[i * mk.was] * mk.wb[i * mk.wbs]);
-                }
-            }
-            if (k > k0) __syncthreads();   // the exchange rows were read for the previous FFT
-            reg_line_fft_v<N, true>(v, p, xl, tw, u);
-        }
-        if (valid) {
-            const float a0 = after ? mk.wa[0] : 1.f;
-            float2* y = Y + z * ystride + k1 + P1 * k2;
-#pragma unroll
-            for (int j = 0; j < Ge::M; ++j)
-#pragma unroll
-                for (int kk = 0; kk < N2; ++kk) {
-                    const float2 w = u[j * N2 + kk];
-                    y[((p + N2 * j) + N1 * kk) * s3] = after ? c_scale(w, a0) : w;
-                }
-        }
-    }
-}
-
-// Synthesis line pass over a chunk's segments: per segment FFT_3 of every item
-// times its mask, summed in float32 over the segment's terms, then added into
-// the accumulator with one Kahan step against the compensation grid comp: the
-// compensation carries across segments and launches, so the sum over the mask
-// groups of the whole synthesis is compensated
-// (src/transforms/ns_surfacelet.jl:292, 355, 383 accumulate every subband into
-// one spectrum).  CTAs take line blocks of the union box (un) and skip the
-// segments whose box none of their lines meets.  With several accumulators
-// (P.ngrp, blockIdx.z) mask group g goes to accumulator g mod ngrp.
-//
-// A wedge plane constant along axis 3 commutes with the axis-3 FFT, so the
-// items that share plane b (and the group factor) are combined first,
-// sum_p wa_p(k1, k2) Y_pq, and transformed once: with nbq > 0 the segment is
-// nbq plane-b wedges q times whole rows p (item t = p nbq + q); otherwise
-// every item is its own term.  Terms are added in q order.
-template <int N>
-__global__ void __launch_bounds__(256, accum_minb<N>())
-    ns_slab_accum_kernel(const float2* __restrict__ Y, long long ystride, int P1, int s3, BoxMap un,
-                         const __grid_constant__ NSMaskTables tb, const __grid_constant__ Chunk ck, int synth,
-                         float2* acc, float2* comp, const float2* __restrict__ tw, long long ychs, long long achs,
-                         long long agrp) {
-    using Ge = RegGeom<N>;
-    constexpr int N1 = Ge::N1, N2 = Ge::N2, LP = Ge::LP, E = Ge::M * Ge::N2;
-    extern __shared__ float2 xch[];
-    Y += blockIdx.y * ychs;   // channel
-    acc += blockIdx.y * achs + blockIdx.z * agrp;
-    comp += blockIdx.y * achs + blockIdx.z * agrp;
-    const int tid = threadIdx.x;
-    const int lp = tid % LP, p = tid / LP;
-    const int l = blockIdx.x * LP + lp;
-    const bool inl = l < un.nk1 * un.nk2;
-    int k1 = 0, k2 = 0;
-    if (inl) un.k12(l, k1, k2);
-    float2* xl = xch + lp * Ge::XLINE;
-    // a segment's sums: in registers, or (lengths whose registers would spill) in shared memory after the
-    // exchange rows, value q of thread t at [q * 256 + t]
-    constexpr bool kSumsShared = accum_sums_shared<N>();
-    float2 sr[kSumsShared ? 1 : E];
-    float2* ss = xch + LP * Ge::XLINE + tid;
-    auto sum = [&](int q) -> float2& {
-        if constexpr (kSumsShared)
-            return ss[q * Ge::THREADS];
-        else
-            return sr[q];
-    };
-    const int si = tb.h1 * tb.n2;
-    const bool wedge_masks = !(synth && !tb.tight);
-    const float2* yl = Y + k1 + P1 * k2;
-#pragma unroll 1
-    for (int sgi = 0; sgi < ck.nseg; ++sgi) {
-        const ChunkSeg& sg = ck.seg[sgi];
-        if (sg.ord % (int)gridDim.z != (int)blockIdx.z) continue;   // another accumulator's
-        const bool valid = inl && k1 < sg.nk1 && (k2 <= sg.b2 || k2 >= tb.n2 - sg.b2);
-        // (the barrier also keeps the previous segment's exchange reads ahead of this one's writes)
-        if (ck.nseg > 1 && !__syncthreads_or(valid)) continue;
-#pragma unroll
-        for (int q = 0; q < E; ++q) sum(q) = make_float2(0.f, 0.f);
-        // the group factor of the line (group table, bandpass table or the lowpass factors), once for all items
-        float gf[E];
-        {
-            const NSMaskLine m0 = chunk_mask_line(tb, sg, ck.item[sg.i0], k1, k2, synth != 0);
-#pragma unroll
-            for (int j = 0; j < Ge::M; ++j)
-#pragma unroll
-                for (int k = 0; k < N2; ++k) {
-                    const int k3 = (p + N2 * j) + N1 * k;
-                    gf[j * N2 + k] = m0.low ? m0.lowc * m0.lowv[k3] : m0.m[(long long)k3 * si];
-                }
-        }
-        const int nbq = sg.nbq;
-        const int rows = nbq > 0 ? sg.nz / nbq : 1;
-        const int nterms = nbq > 0 ? nbq : sg.nz;
-#pragma unroll 1
-        for (int t = 0; t < nterms; ++t) {
-            const ChunkItem& it0 = ck.item[sg.i0 + t];
-            const bool before = wedge_masks && !sg.low && it0.wa_hi != 2;   // plane a applied before the FFT
-            // the term: sum_p wa_p Y_pq (one item with weight 1 when plane a varies along the line; x 1 is
-            // exact).  The loads of the next item are in flight while the current one is added.
-            const int nt = before ? rows : 1;
-            auto weight = [&](int z) {
-                const ChunkItem& it = ck.item[z];
-                return before ? __ldg(tb.planes + it.wa_off + (it.wa_lo == 0 ? k1 : k2) + it.wa_dlo * k2) : 1.f;
-            };
-            float2 v[N1], yb[N1];
-            const int z0 = sg.i0 + t;
-            float wz = weight(z0);
-            {
-                const float2* yz = yl + z0 * ystride;
-#pragma unroll
-                for (int r = 0; r < N1; ++r) yb[r] = valid ? yz[(long long)(p + N2 * r) * s3] : make_float2(0.f, 0.f);
-            }
-#pragma unroll 1
-            for (int pp = 0; pp < nt; ++pp) {
-                const float az = wz;
-                if constexpr (N1 <= 16) {
-                    // a second buffer for the next item's loads (long lines would spill it)
-                    float2 cur[N1];
-#pragma unroll
-                    for (int r = 0; r < N1; ++r) cur[r] = yb[r];
-                    if (pp + 1 < nt) {
-                        const int z = z0 + (pp + 1) * nbq;
-                        const float2* yz = yl + z * ystride;
-                        wz = weight(z);
-#pragma unroll
-                        for (int r = 0; r < N1; ++r)
-                            yb[r] = valid ? yz[(long long)(p + N2 * r) * s3] : make_float2(0.f, 0.f);
-                    }
-#pragma unroll
-                    for (int r = 0; r < N1; ++r) v[r] = pp == 0 ? c_scale(cur[r], az) : c_fma(cur[r], az, v[r]);
-                } else {
-#pragma unroll
-                    for (int r = 0; r < N1; ++r) v[r] = pp == 0 ? c_scale(yb[r], az) : c_fma(yb[r], az, v[r]);
-                    if (pp + 1 < nt) {
-                        const int z = z0 + (pp + 1) * nbq;
-                        const float2* yz = yl + z * ystride;
-                        wz = weight(z);
-#pragma unroll
-                        for (int r = 0; r < N1; ++r)
-                            yb[r] = valid ? yz[(long long)(p + N2 * r) * s3] : make_float2(0.f, 0.f);
-                    }
-                }
-            }
-            float2 u[E];
-            if (t > 0) __syncthreads();   // the exchange rows were read for the previous term
-            reg_line_fft_v<N, false>(v, p, xl, tw, u);
-            // the term's first item carries plane b and the group factor
-            const NSMaskLine mk = chunk_mask_line(tb, sg, it0, k1, k2, synth != 0);
-            const bool wedges = !(mk.low || mk.plain);
-#pragma unroll
-            for (int j = 0; j < Ge::M; ++j)
-#pragma unroll
-                for (int k = 0; k < N2; ++k) {
-                    const int k3 = (p + N2 * j) + N1 * k;
-                    const float g = gf[j * N2 + k];
-                    const float m = !wedges ? g : (before ? g * mk.wb[k3 * mk.wbs] : g * (mk.wa[k3 * mk.was] * mk.wb[k3 * mk.wbs]));
-                    float2& tsum = sum(j * N2 + k);
-                    tsum = make_float2(fmaf(u[j * N2 + k].x, m, tsum.x), fmaf(u[j * N2 + k].y, m, tsum.y));
-                }
-        }
-        if (valid) {
-            float2* a = acc + k1 + P1 * k2;
-            float2* ca = comp + k1 + P1 * k2;
-#pragma unroll
-            for (int j = 0; j < Ge::M; ++j)
-#pragma unroll
-                for (int k = 0; k < N2; ++k) {
-                    const long long o = (long long)((p + N2 * j) + N1 * k) * s3;
-                    float2 sv = a[o], cv = ca[o];
-                    kahan_add(sv, cv, sum(j * N2 + k));
-                    a[o] = sv;
-                    ca[o] = cv;
-                }
-        }
-    }
-}
-
 bool slab_len(int n) { return n == 64 || n == 96 || n == 128 || n == 160 || n == 256; }
 
 int slab_pitch(int h1) { return slab_pitch_c(h1); }
@@ -575,8 +310,12 @@ int acc_groups(const NSPlan& P, const float2* acc) {
 template <int KIND>
 void launch_slab(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char* tag) {
     const int na = P.dims[0], nb = P.dims[1];
-    if (P.mixed)
+    if (P.mixed) {
+        if (any_slab_fits(P))
+            return (KIND == 0 ? launch_any_slab_fwd : KIND == 1 ? launch_any_slab_inv : launch_any_slab_shrink)(P, a, st,
+                                                                                                              tag);
         return (KIND == 0 ? launch_mix_slab_fwd : KIND == 1 ? launch_mix_slab_inv : launch_mix_slab_shrink)(P, a, st, tag);
+    }
     if (slab_cluster_supported(na, nb)) {
         if (!launch_slab_cluster(KIND, na, nb, a, P.sms, st, tag)) throw ArgError("no slab kernel for this size");
         return;
@@ -588,27 +327,6 @@ void launch_slab(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char
 template <bool INV, class Load, class Store>
 void line3(const NSPlan& P, const Load& ld, const Store& so, int nlines, int nz, cudaStream_t st, const char* tag) {
     launch_line<INV>(*P.ffts.at(P.dims[2]), ld, so, nlines, nz, true, st, tag);
-}
-
-template <int N>
-void launch_slab_accum(const NSPlan& P, const Chunk& ck, int synth, float2* acc, float2* comp, int nch, long long ychs,
-                       cudaStream_t st) {
-    using Ge = RegGeom<N>;
-    static bool configured = false;
-    if (!configured) {
-        cuda_check(cudaFuncSetAttribute(ns_slab_accum_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)accum_smem<N>()),
-                   "cudaFuncSetAttribute");
-        configured = true;
-    }
-    const NSBox un = union_box(ck);
-    dim3 grid((un.nk1 * un.nk2 + Ge::LP - 1) / Ge::LP, nch, acc_groups(P, acc));
-    int tok = prof_begin("ns_slab_accum_axis3", st);
-    ns_slab_accum_kernel<N><<<grid, Ge::THREADS, accum_smem<N>(), st>>>(
-        P.work.as<float2>(), P.SP, P.P1, P.P1 * P.dims[1], box_map(P, un), P.tb, ck, synth, acc, comp,
-        P.ffts.at(P.dims[2])->sh.tw, ychs, P.SP, (long long)P.nch * P.SP);
-    prof_end(tok, st);
-    cuda_check(cudaGetLastError(), "ns_slab_accum_kernel launch");
 }
 
 thread_local bool t_concurrent = false;
@@ -666,27 +384,6 @@ int choose_mask_tiles(const NSPlan& P, const Chunk& ck, int lp, int nch, MaskTil
     return ctas;
 }
 
-template <int N>
-void launch_mask_group(const NSPlan& P, const float2* X, const Chunk& ck, int synth, int nch, long long xchs,
-                       long long ychs, cudaStream_t st) {
-    using Ge = RegGeom<N>;
-    static bool configured = false;
-    if (!configured) {
-        cuda_check(cudaFuncSetAttribute(ns_slab_mask_group_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)Ge::SMEM),
-                   "cudaFuncSetAttribute");
-        configured = true;
-    }
-    MaskTiles tl;
-    const int ctas = choose_mask_tiles(P, ck, Ge::LP, nch, tl);
-    int tok = prof_begin("ns_slab_mask_axis3", st);
-    ns_slab_mask_group_kernel<N><<<dim3(ctas, nch), Ge::THREADS, Ge::SMEM, st>>>(
-        X, P.P1, P.P1 * P.dims[1], P.tb, ck, tl, synth, P.work.as<float2>(), P.SP, P.ffts.at(P.dims[2])->sh.tw, xchs,
-        ychs);
-    prof_end(tok, st);
-    cuda_check(cudaGetLastError(), "ns_slab_mask_group_kernel launch");
-}
-
 // Channels: complex volumes run their two real channels in the same launches
 // (spectra and intermediates one block per channel, the volume's channels
 // interleaved floats), with each channel's arithmetic that of a real volume.
@@ -741,24 +438,12 @@ void slab_mask_pass(NSPlan& P, const float2* X, const Chunk& ck, bool synth_mask
     prof_bytes("ns_slab_mask_axis3", nch * (1.5 * segs_bytes(P, ck) + items_bytes(P, ck)));
     const int sy = synth_masks ? 1 : 0;
     const long long xc = P.SP, yc = ych_stride(P);
-    if (P.mixed) {
-        MaskTiles tl;
-        choose_mask_tiles(P, ck, mix_axis3_lines(P), nch, tl);
-        int tok = prof_begin("ns_slab_mask_axis3", st);
-        launch_mix_mask(P, X, ck, tl, sy, P.work.as<float2>(), nch, xc, yc, st);
-        prof_end(tok, st);
-        return;
-    }
-    switch (P.dims[2]) {
-        case 16: launch_mask_group<16>(P, X, ck, sy, nch, xc, yc, st); return;
-        case 32: launch_mask_group<32>(P, X, ck, sy, nch, xc, yc, st); return;
-        case 64: launch_mask_group<64>(P, X, ck, sy, nch, xc, yc, st); return;
-        case 96: launch_mask_group<96>(P, X, ck, sy, nch, xc, yc, st); return;
-        case 128: launch_mask_group<128>(P, X, ck, sy, nch, xc, yc, st); return;
-        case 160: launch_mask_group<160>(P, X, ck, sy, nch, xc, yc, st); return;
-        case 256: launch_mask_group<256>(P, X, ck, sy, nch, xc, yc, st); return;
-    }
-    throw ArgError("no register line pass for axis 3 of this size");
+    MaskTiles tl;
+    const bool any = axis3_len(P.dims[2]);
+    choose_mask_tiles(P, ck, any ? axis3_lines(P.dims[2]) : mix_axis3_lines(P), nch, tl);
+    int tok = prof_begin("ns_slab_mask_axis3", st);
+    (any ? launch_axis3_mask : launch_mix_mask)(P, X, ck, tl, sy, P.work.as<float2>(), nch, xc, yc, st);
+    prof_end(tok, st);
 }
 
 // The synthesis axis-3 pass of a chunk from Y into acc + ch SP,
@@ -769,23 +454,11 @@ void slab_accum_pass(NSPlan& P, const Chunk& ck, bool analysis_masks, float2* ac
     prof_bytes("ns_slab_accum_axis3", nch * (items_bytes(P, ck) + 4.5 * segs_bytes(P, ck)));
     const int sy = analysis_masks ? 0 : 1;
     const long long yc = ych_stride(P);
-    if (P.mixed) {
-        int tok = prof_begin("ns_slab_accum_axis3", st);
-        launch_mix_accum(P, ck, box_map(P, union_box(ck)), sy, P.work.as<float2>(), acc, comp, nch, acc_groups(P, acc),
-                         yc, st);
-        prof_end(tok, st);
-        return;
-    }
-    switch (P.dims[2]) {
-        case 16: launch_slab_accum<16>(P, ck, sy, acc, comp, nch, yc, st); return;
-        case 32: launch_slab_accum<32>(P, ck, sy, acc, comp, nch, yc, st); return;
-        case 64: launch_slab_accum<64>(P, ck, sy, acc, comp, nch, yc, st); return;
-        case 96: launch_slab_accum<96>(P, ck, sy, acc, comp, nch, yc, st); return;
-        case 128: launch_slab_accum<128>(P, ck, sy, acc, comp, nch, yc, st); return;
-        case 160: launch_slab_accum<160>(P, ck, sy, acc, comp, nch, yc, st); return;
-        case 256: launch_slab_accum<256>(P, ck, sy, acc, comp, nch, yc, st); return;
-    }
-    throw ArgError("no register line pass for axis 3 of this size");
+    int tok = prof_begin("ns_slab_accum_axis3", st);
+    (axis3_len(P.dims[2]) ? launch_axis3_accum : launch_mix_accum)(P, ck, box_map(P, union_box(ck)), sy,
+                                                                   P.work.as<float2>(), acc, comp, nch,
+                                                                   acc_groups(P, acc), yc, st);
+    prof_end(tok, st);
 }
 
 // Analysis of items [i0, i0 + nz) (one chunk) from X (+ ch SP) into volumes at

@@ -38,3 +38,27 @@ def test_line_lengths_match_oracle(sfl, n, axis, pipeline):
         assert np.linalg.norm(sfl.to_host(b) - r) <= TOL * max(np.linalg.norm(r), 1e-3 * np.linalg.norm(x))
     y = sfl.to_host(sfl.hourglass_reconstruct(ws, bands))
     assert np.linalg.norm(y - x) <= TOL * np.linalg.norm(x)
+
+
+# the lengths compiled for the slab and axis-3 passes: products of two radices up to 16
+TWO_RADIX = [n for n in range(16, 257) if any(n % a == 0 and 2 <= n // a <= 16 for a in range(2, 17))]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", TWO_RADIX)
+def test_two_radix_lengths_match_oracle(sfl, n):
+    for axis in range(3):
+        dims = [18, 21, 16]
+        dims[axis] = n
+        dims = tuple(dims)
+        x = np.random.default_rng(n + axis).standard_normal(dims).astype(np.float32)
+        ws = sfl.make_workspace(sfl.HourglassFB(bernstein_order=6), "float32", dims)
+        assert ws.tuning()[0] == "mixed"
+        bands = sfl.hourglass_decompose(ws, sfl.to_device(x))
+        for b, r in zip(bands, N.hourglass_decompose(x, dims, 6, 1)):
+            assert np.linalg.norm(sfl.to_host(b) - r) <= TOL * max(np.linalg.norm(r), 1e-3 * np.linalg.norm(x))
+        y = sfl.to_host(sfl.hourglass_reconstruct(ws, bands))
+        assert np.linalg.norm(y - x) <= TOL * np.linalg.norm(x)
+        # the denoiser at threshold 0 is the round trip, bit for bit
+        z = sfl.to_host(sfl.denoise(ws, sfl.to_device(x), np.zeros(3, np.float32)))
+        assert np.array_equal(z, y)
