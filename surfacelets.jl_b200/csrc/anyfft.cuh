@@ -93,12 +93,22 @@ __device__ __forceinline__ void any_block_fft(float2 (&v)[AnyLine<N>::N1], int p
     for (int j = 0; j < G::M; ++j) {
         const int m = p + N2 * j;
         float2 w[N2];
+        const float2* xm = xl + (G::has(p, j) ? m * G::XROW : 0);
 #pragma unroll
-        for (int q = 0; q < N2; ++q) w[q] = G::has(p, j) ? xl[m * G::XROW + q] : make_float2(0.f, 0.f);
+        for (int q = 0; q < N2; ++q) w[q] = xm[q];
         RegDft<N2, INV>::run(w);
 #pragma unroll
         for (int k = 0; k < N2; ++k) u[j * N2 + k] = w[k];
     }
+}
+
+// Lane layout of column pairs (lines 2 P1 slots apart, P1 = 2 mod 4): with four
+// lines a warp the two lines of a half warp are two apart, so that their slots
+// fall on disjoint banks.
+template <int N>
+__device__ __forceinline__ int any_pair_line(int s) {
+    if (AnyLine<N>::N2 == 8) return s == 1 ? 2 : (s == 2 ? 1 : s);
+    return s;
 }
 
 // Twiddles of a warp line FFT rearranged as tw2[m N2 + p] = w_N^{p m}.
@@ -142,9 +152,10 @@ __device__ __forceinline__ void any_warp_fft(float2 (&v)[AnyLine<N>::N1], int p,
 #pragma unroll
     for (int j = 0; j < L::M; ++j) {
         float2 w[N2];
-        const bool act = valid && L::has(p, j);
+        // lanes without a line or an output read the first slots and are dropped by the caller
+        const float2* rj = L::has(p, j) ? rb + stride * N2 * N2 * j : base;
 #pragma unroll
-        for (int q = 0; q < N2; ++q) w[q] = act ? rb[xo[q] + stride * N2 * N2 * j] : make_float2(0.f, 0.f);
+        for (int q = 0; q < N2; ++q) w[q] = rj[xo[q]];
         RegDft<N2, INV>::run(w);
 #pragma unroll
         for (int k = 0; k < N2; ++k) u[j * N2 + k] = w[k];

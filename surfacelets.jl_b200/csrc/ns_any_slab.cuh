@@ -40,11 +40,15 @@ __device__ __noinline__ void any_rows(int so, int P1, int rows, int b2, int k2hi
         const bool valid = s < L::LPW && k1 < rows;
         float2* row = S + (valid ? k1 : 0);
         float2 v[N1], u[L::E];
+        if (!INV || b2 >= N) {
 #pragma unroll
-        for (int r = 0; r < N1; ++r) {
-            const int k2 = p + N2 * r;
-            const bool in = valid && (!INV || k2 <= b2 || k2 >= k2hi);
-            v[r] = in ? row[P1 * k2] : make_float2(0.f, 0.f);
+            for (int r = 0; r < N1; ++r) v[r] = row[P1 * (p + N2 * r)];
+        } else {
+#pragma unroll
+            for (int r = 0; r < N1; ++r) {
+                const int k2 = p + N2 * r;
+                v[r] = k2 <= b2 || k2 >= k2hi ? row[P1 * k2] : make_float2(0.f, 0.f);
+            }
         }
         any_warp_fft<N, INV>(v, p, valid, tw2, row, P1, u);
 #pragma unroll
@@ -56,6 +60,9 @@ __device__ __noinline__ void any_rows(int so, int P1, int rows, int b2, int k2hi
     }
 }
 
+// The column of zeros, behind the slab's spare column.
+__device__ __forceinline__ const float2* any_zero(int so, int P1, int n2) { return any_sm + so + P1 * (n2 + 1); }
+
 // The next unit's box columns, requested as soon as their pairs are transformed.
 struct AnyNext {
     const float2* src;   // null: no next unit
@@ -64,25 +71,32 @@ struct AnyNext {
     int bar;             // offset of the mbarrier
 };
 
-// The full spectrum of (column 2l) + i (column 2l + 1) at v[r] = Z[p + N2 r]: rows
-// k1 >= nk1 are zero, and the missing column of an odd count.
+// The full spectrum of (column ca) + i (column cb) at v[r] = Z[p + N2 r]: rows
+// k1 >= nk1 are zero; cb is a column of zeros where an odd count's last column
+// has no partner.
 template <int N>
-__device__ __forceinline__ void any_load_pair(float2 (&v)[AnyLine<N>::N1], const float2* ca, int P1, int nk1, int p,
-                                              bool valid, bool two) {
-#pragma unroll
-    for (int r = 0; r < AnyLine<N>::N1; ++r) {
-        const int i = p + AnyLine<N>::N2 * r;
-        const int k = 2 * i <= N ? i : N - i;
-        float2 A = make_float2(0.f, 0.f), B = make_float2(0.f, 0.f);
-        if (valid && k < nk1) {
-            A = ca[k];
-            if (two) B = ca[P1 + k];
-        }
+__device__ __forceinline__ void any_load_pair(float2 (&v)[AnyLine<N>::N1], const float2* ca, const float2* cb, int nk1,
+                                              int p) {
+    auto fold = [&](float2& z, int i, int k, float2 A, float2 B) {
         if (k == 0 || 2 * k == N) {
             A.y = 0.f;
             B.y = 0.f;
         }
-        v[r] = 2 * i <= N ? make_float2(A.x - B.y, A.y + B.x) : make_float2(A.x + B.y, B.x - A.y);
+        z = 2 * i <= N ? make_float2(A.x - B.y, A.y + B.x) : make_float2(A.x + B.y, B.x - A.y);
+    };
+    if (nk1 == N / 2 + 1) {
+#pragma unroll
+        for (int r = 0; r < AnyLine<N>::N1; ++r) {
+            const int i = p + AnyLine<N>::N2 * r, k = 2 * i <= N ? i : N - i;
+            fold(v[r], i, k, ca[k], cb[k]);
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < AnyLine<N>::N1; ++r) {
+            const int i = p + AnyLine<N>::N2 * r, k = 2 * i <= N ? i : N - i;
+            const bool in = k < nk1;
+            fold(v[r], i, k, in ? ca[k] : make_float2(0.f, 0.f), in ? cb[k] : make_float2(0.f, 0.f));
+        }
     }
 }
 
@@ -99,11 +113,11 @@ __device__ __forceinline__ void any_put_natural(const float2 (&u)[AnyLine<N>::E]
 }
 
 // C2R along axis 1 of columns 2l and 2l + 1 as one complex line, scaled, into
-// two columns of a real slab (element stride es); rows k1 >= nk1 are zero, and
+// two columns of a real slab (element stride ES); rows k1 >= nk1 are zero, and
 // the missing column of an odd count.
-template <int N>
-__device__ __noinline__ void any_cols_inv(int so, int P1, int nk1, int n2, int to, float* out, int es, float scale,
-                                          AnyNext nx) {
+template <int N, int ES>
+__device__ __noinline__ void any_cols_inv(int so, int P1, int nk1, int n2, int to, float* out, float scale,
+                                          const AnyNext& nx) {
     float2* const S = any_sm + so;
     const float2* const tw2 = any_sm + to;
     using L = AnyLine<N>;
@@ -112,11 +126,11 @@ __device__ __noinline__ void any_cols_inv(int so, int P1, int nk1, int n2, int t
     const int s = lane / N2, p = lane - s * N2, npairs = (n2 + 1) / 2;
 #pragma unroll 1
     for (int l0 = warp * L::LPW; l0 < npairs; l0 += step) {
-        const int l = l0 + s;
+        const int l = l0 + any_pair_line<N>(s);
         const bool valid = s < L::LPW && l < npairs, two = valid && 2 * l + 1 < n2;
         float2* ca = S + P1 * (2 * (valid ? l : 0));
         float2 v[N1], u[L::E];
-        any_load_pair<N>(v, ca, P1, nk1, p, valid, two);
+        any_load_pair<N>(v, ca, two ? ca + P1 : any_zero(so, P1, n2), nk1, p);
         any_warp_fft<N, true>(v, p, valid, tw2, ca, 1, u);
         if (nx.src) {
             fence_proxy_async();
@@ -128,17 +142,16 @@ __device__ __noinline__ void any_cols_inv(int so, int P1, int nk1, int n2, int t
                 bulk_load(S + P1 * k2, nx.src + P1 * k2, nx.bytes, bar);
             }
         }
-        float* oa = out + (2 * (valid ? l : 0)) * N * es;
-        float* ob = oa + N * es;
+        float* oa = out + ((2 * (valid ? l : 0)) * N + p) * ES;
+        float* ob = oa + N * ES;
 #pragma unroll
         for (int j = 0; j < L::M; ++j)
             if (valid && L::has(p, j)) {
 #pragma unroll
                 for (int k = 0; k < N2; ++k) {
-                    const int i = ((p + N2 * j) + N1 * k) * es;
                     const float2 x = c_scale(u[j * N2 + k], scale);
-                    oa[i] = x.x;
-                    if (two) ob[i] = x.y;
+                    oa[(N2 * j + N1 * k) * ES] = x.x;
+                    if (two) ob[(N2 * j + N1 * k) * ES] = x.y;
                 }
             }
     }
@@ -173,9 +186,9 @@ __device__ __forceinline__ void any_unpack(float2* ca, int P1, int nk1, int p, b
     }
 }
 
-// R2C along axis 1 of columns 2l and 2l + 1 of a real slab (element stride es).
-template <int N>
-__device__ __noinline__ void any_cols_fwd(int so, int P1, int nk1, int n2, int to, const float* in, int es) {
+// R2C along axis 1 of columns 2l and 2l + 1 of a real slab (element stride ES).
+template <int N, int ES>
+__device__ __noinline__ void any_cols_fwd(int so, int P1, int nk1, int n2, int to, const float* in) {
     float2* const S = any_sm + so;
     const float2* const tw2 = any_sm + to;
     using L = AnyLine<N>;
@@ -184,16 +197,16 @@ __device__ __noinline__ void any_cols_fwd(int so, int P1, int nk1, int n2, int t
     const int s = lane / N2, p = lane - s * N2, npairs = (n2 + 1) / 2;
 #pragma unroll 1
     for (int l0 = warp * L::LPW; l0 < npairs; l0 += step) {
-        const int l = l0 + s;
+        const int l = l0 + any_pair_line<N>(s);
         const bool valid = s < L::LPW && l < npairs, two = valid && 2 * l + 1 < n2;
-        const float* ia = in + (2 * (valid ? l : 0)) * N * es;
-        const float* ib = ia + (two ? N * es : 0);
+        const float* ia = in + ((2 * (valid ? l : 0)) * N + p) * ES;
+        const float* ib = ia + (two ? N * ES : 0);
         float2 v[N1], u[L::E];
 #pragma unroll
-        for (int r = 0; r < N1; ++r) {
-            const int i = (p + N2 * r) * es;
-            v[r] = make_float2(ia[i], ib[i]);
-            if (!two) v[r].y = 0.f;
+        for (int r = 0; r < N1; ++r) v[r] = make_float2(ia[N2 * r * ES], ib[N2 * r * ES]);
+        if (!two) {   // an odd count's last column has no partner
+#pragma unroll
+            for (int r = 0; r < N1; ++r) v[r].y = 0.f;
         }
         float2* ca = S + P1 * (2 * (valid ? l : 0));
         any_warp_fft<N, false>(v, p, valid, tw2, ca, 1, u);
@@ -215,11 +228,11 @@ __device__ __noinline__ void any_cols_shrink(int so, int P1, int nk1, int n2, in
     const int s = lane / N2, p = lane - s * N2, npairs = (n2 + 1) / 2;
 #pragma unroll 1
     for (int l0 = warp * L::LPW; l0 < npairs; l0 += step) {
-        const int l = l0 + s;
+        const int l = l0 + any_pair_line<N>(s);
         const bool valid = s < L::LPW && l < npairs, two = valid && 2 * l + 1 < n2;
         float2* ca = S + P1 * (2 * (valid ? l : 0));
         float2 v[N1], u[L::E];
-        any_load_pair<N>(v, ca, P1, nk1, p, valid, two);
+        any_load_pair<N>(v, ca, two ? ca + P1 : any_zero(so, P1, n2), nk1, p);
         any_warp_fft<N, true>(v, p, valid, tw2, ca, 1, u);
 #pragma unroll
         for (int j = 0; j < L::M; ++j)
@@ -282,18 +295,18 @@ constexpr int kAnyThreads = 512;
 // Values before the slab: both axes' twiddles, rounded up so that the slab
 // starts 16-byte aligned.
 __host__ __device__ inline int any_tw_values(int n1, int n2) { return (n1 + n2 + 1) & ~1; }
-// The slab with one spare column (the exchange slots of an odd count's last
-// column), then the mbarrier.
+// The slab, a spare column (the exchange slots of an odd count's last column)
+// and a column of zeros, then the mbarrier.
 inline size_t any_smem(int n1, int n2, int P1) {
-    return sizeof(float2) * ((size_t)any_tw_values(n1, n2) + (size_t)P1 * (n2 + 1)) + 16;
+    return sizeof(float2) * ((size_t)any_tw_values(n1, n2) + (size_t)P1 * (n2 + 2)) + 16;
 }
 
 // KIND: 0 the forward slab pass, 1 the inverse, 2 the denoiser's shrink pass.
 // One CTA a unit (channel, item, n3), striding over the launch's units.
-template <int KIND>
+template <int KIND, int ES>
 __global__ void __launch_bounds__(kAnyThreads, 2)
     ns_any_slab_kernel(const __grid_constant__ SlabArgs a, const int n1, const int n2) {
-    const int P1 = a.P1, so = any_tw_values(n1, n2), bo = so + P1 * (n2 + 1);
+    const int P1 = a.P1, so = any_tw_values(n1, n2), bo = so + P1 * (n2 + 2);
     float2* S = any_sm + so;
     uint64_t* bar = reinterpret_cast<uint64_t*>(any_sm + bo);
     uint32_t phase = 0;
@@ -309,6 +322,7 @@ __global__ void __launch_bounds__(kAnyThreads, 2)
         SFL_ANY_LENGTHS(SFL_ANY_CASE)
 #undef SFL_ANY_CASE
     }
+    for (int i = threadIdx.x; i < P1; i += blockDim.x) S[P1 * (n2 + 1) + i] = make_float2(0.f, 0.f);
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         fence_barrier_init();
@@ -328,11 +342,11 @@ __global__ void __launch_bounds__(kAnyThreads, 2)
         const int z = ur / a.n3, s3 = ur - z * a.n3;
         const ChunkItem& it = a.ck.item[z];
         const int nk1 = it.nk1, b2 = it.b2, k2hi = n2 - (it.nk2 - b2 - 1);
-        float* vol = a.vol + ch + a.vol_off(z) + (long long)s3 * PLANE * a.es;
+        float* vol = a.vol + ch + a.vol_off(z) + (long long)s3 * PLANE * ES;
         if constexpr (KIND == 0) {
             switch (n1) {
 #define SFL_ANY_CASE(N_) \
-    case N_: any_cols_fwd<N_>(so, P1, nk1, n2, 0, vol, a.es); break;
+    case N_: any_cols_fwd<N_, ES>(so, P1, nk1, n2, 0, vol); break;
                 SFL_ANY_LENGTHS(SFL_ANY_CASE)
 #undef SFL_ANY_CASE
             }
@@ -388,7 +402,7 @@ __global__ void __launch_bounds__(kAnyThreads, 2)
             __syncthreads();
             switch (n1) {
 #define SFL_ANY_CASE(N_) \
-    case N_: any_cols_inv<N_>(so, P1, nk1, n2, 0, vol, a.es, a.scale, nx); break;
+    case N_: any_cols_inv<N_, ES>(so, P1, nk1, n2, 0, vol, a.scale, nx); break;
                 SFL_ANY_LENGTHS(SFL_ANY_CASE)
 #undef SFL_ANY_CASE
             }
@@ -423,9 +437,9 @@ inline int any_warps(int n1, int n2, size_t smem) {
     return w;
 }
 
-template <int KIND>
-void launch_any_slab(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char* tag) {
-    auto kern = ns_any_slab_kernel<KIND>;
+template <int KIND, int ES>
+void launch_any_slab_es(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char* tag) {
+    auto kern = ns_any_slab_kernel<KIND, ES>;
     static bool configured = false;
     if (!configured) {
         cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmemOneCta),
@@ -443,6 +457,14 @@ void launch_any_slab(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const 
     kern<<<grid, threads, smem, st>>>(a, n1, n2);
     prof_end(tok, st);
     cuda_check(cudaGetLastError(), "ns_any_slab_kernel launch");
+}
+
+template <int KIND>
+void launch_any_slab(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char* tag) {
+    if (KIND == 2 || a.es == 1)
+        launch_any_slab_es<KIND, 1>(P, a, st, tag);
+    else
+        launch_any_slab_es<KIND, 2>(P, a, st, tag);
 }
 
 }  // namespace

@@ -598,7 +598,7 @@ void ns_merge_groups(NSPlan& P, int ch, float2* A, float2* C, cudaStream_t st) {
 // several accumulators, summed by the inverse FFT's first pass.
 int ns_slab_groups(const NSPlan& P) {
     const long long lines = (long long)P.h1 * P.dims[1];
-    return lines <= 5000 ? 4 : (lines <= 10000 ? 2 : 1);
+    return lines <= 3000 ? 4 : (lines <= 10000 ? 2 : 1);
 }
 
 void ns_use_mixed(NSPlan& P) {
