@@ -17,10 +17,10 @@
 #include <cmath>
 #include <cstring>
 
+#include "anyfft.cuh"
 #include "mixpass.cuh"
 #include "plan.h"
 #include "regpass.cuh"
-#include "slab_core.cuh"
 
 namespace sfl {
 
@@ -259,6 +259,9 @@ struct IrcPlaneJob {
     int hd[3];
     const float* V;   // analysis: the hourglass mask V_K and the subband scale s
     float s;
+    // the transposes: the stages' filters conjugated, and the analysis form loads the adjoint of the Hermitian sum
+    // (herm_gather_kernel) instead of the masked spectrum; nK is the full length of axis K
+    int adjoint, nK;
     IrcPlaneStages sg;
     // the block FFTs along the two transverse axes, fused: segment lengths (0: run separately) and the
     // twiddle tables w_bs^k of those lengths
@@ -276,78 +279,79 @@ struct IrcPlaneJobs {
 // along either axis of the plane are free of bank conflicts.
 __host__ __device__ inline int irc_plane_pitch(int a1) { return a1 % 4 == 0 ? a1 + 2 : a1; }
 
-// Block FFT lengths the plane pass runs itself (register line FFTs of at most
-// 16 values a thread, within the 64 registers of a 1024-thread CTA).
-__host__ __device__ inline bool irc_plane_block_len(int n) { return n == 16 || n == 32 || n == 64 || n == 128; }
+// Block FFT lengths the plane pass runs itself: those with a compile-time line
+// FFT (anyfft.cuh; at most 16 values a thread, within the 64 registers of a
+// 1024-thread CTA).
+__host__ inline bool irc_plane_block_len(int n) { return any_len(n); }
 
-// The segmented FFTs of the plane along one transverse axis: segments of N
-// points (the block length), unnormalized, inverse or forward.  Lines of a
-// warp sit on consecutive rows (along the first axis) or consecutive columns
-// (along the second), so their slots fall on distinct banks.
+extern __shared__ __align__(16) float2 irc_sm[];
+
+// The segmented FFTs of the plane (at the start of shared memory) along one
+// transverse axis: segments of N points (the block length), unnormalized,
+// inverse or forward, twiddles at offset `to`.  Lines of a warp sit on
+// consecutive rows (along the first axis) or consecutive columns (along the
+// second), so their slots fall on distinct banks.  A function of its own per
+// length: inlined, the 82 lengths would make one kernel too large to compile.
 template <int N, bool INV>
-__device__ void irc_plane_seg_fft(float2* pl, int ap, int a1, int a2, bool along1, const float2* tw2s) {
-    using LN = SlabLine<N>;
+__device__ __noinline__ void irc_plane_seg_fft(int ap, int a1, int a2, bool along1, int to) {
+    using LN = AnyLine<N>;
     constexpr int N1 = LN::N1, N2 = LN::N2;
+    float2* const pl = irc_sm;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int p = lane & (N2 - 1), sl = lane / N2;
+    const int sl = lane / N2, p = lane - sl * N2;
     const int nseg = (along1 ? a1 : a2) / N;
     const int nl = (along1 ? a2 : a1) * nseg;
-    for (int b0 = 0; b0 < nl; b0 += nwarps * LN::LPW) {
-        if (b0 + warp * LN::LPW >= nl) continue;   // warp-uniform
-        const int line = b0 + warp * LN::LPW + sl;
-        const bool valid = line < nl;
+#pragma unroll 1
+    for (int b0 = warp * LN::LPW; b0 < nl; b0 += nwarps * LN::LPW) {
+        const int line = b0 + sl;
+        const bool valid = sl < LN::LPW && line < nl;
         const int li = valid ? line : 0;
         float2* base;
         int stride;
         if (along1) {
-            const int o2 = li % a2, seg = li / a2;
-            base = pl + (long long)o2 * ap + seg * N;
+            const int seg = li / a2, o2 = li - seg * a2;
+            base = pl + o2 * ap + seg * N;
             stride = 1;
         } else {
-            const int o1 = li % a1, seg = li / a1;
-            base = pl + o1 + (long long)seg * N * ap;
+            const int seg = li / a1, o1 = li - seg * a1;
+            base = pl + o1 + seg * N * ap;
             stride = ap;
         }
-        float2 v[N1];
+        float2 v[N1], u[LN::E];
 #pragma unroll
-        for (int r = 0; r < N1; ++r) v[r] = valid ? base[stride * (p + N2 * r)] : make_float2(0.f, 0.f);
-        warp_line_fft_rs<N, INV>(v, p, valid, tw2s, base, stride);
-        if (valid) {
+        for (int r = 0; r < N1; ++r) v[r] = base[stride * (p + N2 * r)];
+        any_warp_fft<N, INV>(v, p, valid, irc_sm + to, base, stride, u);
 #pragma unroll
-            for (int j = 0; j < LN::M; ++j)
+        for (int j = 0; j < LN::M; ++j)
+            if (valid && LN::has(p, j)) {
 #pragma unroll
-                for (int k = 0; k < N2; ++k) base[stride * ((p + N2 * j) + N1 * k)] = v[j * N2 + k];
-        }
+                for (int k = 0; k < N2; ++k) base[stride * ((p + N2 * j) + N1 * k)] = u[j * N2 + k];
+            }
     }
 }
 
 template <bool INV>
-__device__ void irc_plane_block_ffts(float2* pl, int ap, int a1, int a2, int bs, bool along1, const float2* tw2s) {
+__device__ __forceinline__ void irc_plane_block_ffts(int ap, int a1, int a2, int bs, bool along1, int to) {
     switch (bs) {
-        case 16: irc_plane_seg_fft<16, INV>(pl, ap, a1, a2, along1, tw2s); break;
-        case 32: irc_plane_seg_fft<32, INV>(pl, ap, a1, a2, along1, tw2s); break;
-        case 64: irc_plane_seg_fft<64, INV>(pl, ap, a1, a2, along1, tw2s); break;
-        case 128: irc_plane_seg_fft<128, INV>(pl, ap, a1, a2, along1, tw2s); break;
+#define SFL_ANY_CASE(N_) \
+    case N_: irc_plane_seg_fft<N_, INV>(ap, a1, a2, along1, to); break;
+        SFL_ANY_LENGTHS(SFL_ANY_CASE)
+#undef SFL_ANY_CASE
     }
 }
 
-template <int N>
-__device__ void irc_plane_twiddles(float2* tw2s, const float2* tw) {
-    load_slab_twiddles<N>(tw2s, tw);
-}
-
-__device__ void irc_plane_load_twiddles(float2* tw2s, const float2* tw, int bs) {
+__device__ __forceinline__ void irc_plane_load_twiddles(float2* tw2s, const float2* tw, int bs) {
     switch (bs) {
-        case 16: irc_plane_twiddles<16>(tw2s, tw); break;
-        case 32: irc_plane_twiddles<32>(tw2s, tw); break;
-        case 64: irc_plane_twiddles<64>(tw2s, tw); break;
-        case 128: irc_plane_twiddles<128>(tw2s, tw); break;
+#define SFL_ANY_CASE(N_) \
+    case N_: any_load_twiddles<N_>(tw2s, tw); break;
+        SFL_ANY_LENGTHS(SFL_ANY_CASE)
+#undef SFL_ANY_CASE
     }
 }
 
 template <bool SYNTH>
 __global__ void __launch_bounds__(kIrcPlaneThreads) irc_plane_kernel(const __grid_constant__ IrcPlaneJobs jobs) {
-    extern __shared__ float2 pl[];
+    float2* const pl = irc_sm;
     int t0 = 0;
     while (t0 + 1 < jobs.n && (int)blockIdx.x >= jobs.job[t0 + 1].first) ++t0;
     const IrcPlaneJob& jb = jobs.job[t0];
@@ -369,6 +373,9 @@ __global__ void __launch_bounds__(kIrcPlaneThreads) irc_plane_kernel(const __gri
     const int kK = blockIdx.x - jb.first;
     const long long base = (long long)kK * sK;
     const long long xbase = (long long)kK * xK;
+    // adjoint of the Hermitian sum: the bins whose mirror lies outside the half grid add its conjugate
+    const bool mirrored = !SYNTH && jb.adjoint && kK > 0 && jb.nK - kK >= nKh;
+    const long long xmir = mirrored ? (long long)(jb.nK - kK) * xK : 0;
     const int tot = a1 * a2;
     const FastDiv fa1((unsigned)a1);
     const int ap = irc_plane_pitch(a1);                  // the plane's row pitch in shared memory
@@ -390,7 +397,12 @@ __global__ void __launch_bounds__(kIrcPlaneThreads) irc_plane_kernel(const __gri
                 const int i2 = (int)fa1.div((unsigned)q), i1 = q - i2 * a1;
                 const long long g = base + i1 * s1 + i2 * s2;
                 if (!SYNTH) {
-                    v[u] = c_scale(X[xbase + i1 * xa + i2 * xb], V[g] * s);
+                    float2 x = X[xbase + i1 * xa + i2 * xb];
+                    if (mirrored) {
+                        const int r1 = i1 ? a1 - i1 : 0, r2 = i2 ? a2 - i2 : 0;
+                        x = c_add(x, c_conj(X[xmir + r1 * xa + r2 * xb]));
+                    }
+                    v[u] = c_scale(x, V[g] * s);
                 } else {
                     v[u] = S[g];
                 }
@@ -408,9 +420,9 @@ __global__ void __launch_bounds__(kIrcPlaneThreads) irc_plane_kernel(const __gri
     __syncthreads();
     if (SYNTH && fused) {
         // subband -> block: the forward block FFTs along both transverse axes, then the stages in reverse
-        irc_plane_block_ffts<false>(pl, ap, a1, a2, jb.bs1, true, tws);
+        irc_plane_block_ffts<false>(ap, a1, a2, jb.bs1, true, (int)(tws - pl));
         __syncthreads();
-        irc_plane_block_ffts<false>(pl, ap, a1, a2, jb.bs2, false, tws + jb.bs1);
+        irc_plane_block_ffts<false>(ap, a1, a2, jb.bs2, false, (int)(tws - pl) + jb.bs1);
         __syncthreads();
     }
     for (int t = 0; t < sg.n; ++t) {
@@ -423,8 +435,13 @@ __global__ void __launch_bounds__(kIrcPlaneThreads) irc_plane_kernel(const __gri
         // the stage's filter row at k_K (over the stage's axis) into shared memory
         const int am = first ? a1 : a2;
         for (int i = threadIdx.x; i < am; i += blockDim.x) {
-            cf[i] = sg.f0[u][kK + (long long)nKh * i];
-            cf[am + i] = sg.f1[u][kK + (long long)nKh * i];
+            float2 f0 = sg.f0[u][kK + (long long)nKh * i], f1 = sg.f1[u][kK + (long long)nKh * i];
+            if (jb.adjoint) {
+                f0.y = -f0.y;
+                f1.y = -f1.y;
+            }
+            cf[i] = f0;
+            cf[am + i] = f1;
         }
         __syncthreads();
         for (int q = threadIdx.x; q < npairs; q += blockDim.x) {
@@ -453,9 +470,9 @@ __global__ void __launch_bounds__(kIrcPlaneThreads) irc_plane_kernel(const __gri
     }
     if (!SYNTH && fused) {
         // block -> subband, first half: the inverse block FFTs along both transverse axes
-        irc_plane_block_ffts<true>(pl, ap, a1, a2, jb.bs1, true, tws);
+        irc_plane_block_ffts<true>(ap, a1, a2, jb.bs1, true, (int)(tws - pl));
         __syncthreads();
-        irc_plane_block_ffts<true>(pl, ap, a1, a2, jb.bs2, false, tws + jb.bs1);
+        irc_plane_block_ffts<true>(ap, a1, a2, jb.bs2, false, (int)(tws - pl) + jb.bs1);
         __syncthreads();
     }
     for (int q = threadIdx.x; q < tot; q += blockDim.x) {
@@ -1059,11 +1076,11 @@ bool irc_plane_fuses(const DecLevelDev& L, int K) {
 }
 
 // One launch of the plane pass over every level's hourglasses whose plane
-// fits (analysis: with the mask on load from the level spectrum; synthesis:
+// fits, or its transpose (analysis: with the mask on load from the level spectrum; synthesis:
 // hourglasses without stages have nothing to do), the finest level's planes
 // first so that the coarser levels' smaller planes fill the last wave.
 template <bool SYNTH>
-void irc_plane_launch_levels(DecPlan& D, cudaStream_t st) {
+void irc_plane_launch_levels(DecPlan& D, cudaStream_t st, bool adjoint = false) {
     IrcPlaneJobs jobs{};
     size_t smem = 0;
     int blocks = 0;
@@ -1094,8 +1111,11 @@ void irc_plane_launch_levels(DecPlan& D, cudaStream_t st) {
             jb.V = L.V[K].as<float>();
             int sb[3];
             for (int d = 0; d < 3; ++d) sb[d] = d == K ? L.n[K] : L.bsize[K][d];
-            jb.s = (float)(1.0 / ((double)sb[0] * sb[1] * sb[2]));
-            jb.sg = irc_plane_stages(L, K, SYNTH);
+            jb.s = adjoint ? 1.0f / 3.0f : (float)(1.0 / ((double)sb[0] * sb[1] * sb[2]));
+            jb.adjoint = adjoint;
+            jb.nK = L.n[K];
+            // a transpose runs the other direction's form with this direction's filters, conjugated
+            jb.sg = irc_plane_stages(L, K, SYNTH != adjoint);
             if (irc_plane_fuses<SYNTH>(L, K)) {
                 const int m1 = K == 0 ? 1 : 0, m2 = K == 2 ? 1 : 2;
                 jb.bs1 = L.bsize[K][m1];
@@ -1108,6 +1128,53 @@ void irc_plane_launch_levels(DecPlan& D, cudaStream_t st) {
         }
     }
     flush();
+}
+
+// The C2R along K of level L's hourglasses into the subbands, those of one
+// length and line layout in one launch; wpair weighs the bins that are not
+// self-conjugate (0.5: the adjoint of the R2C).
+void blocks_c2r(DecPlan& D, DecLevelDev& L, float* c, int es, float wpair, cudaStream_t st) {
+    bool done[3] = {false, false, false};
+    for (int K = 0; K < 3; ++K) {
+        if (done[K]) continue;
+        LoadJobs<RLoadHPair> lj{};
+        StoreJobs<RStoreRPairBlocks> sj{};
+        int nj = 0, pairs = 0;
+        for (int K2 = K; K2 < 3; ++K2) {
+            if (done[K2] || L.n[K2] != L.n[K] || (K2 != 0) != (K != 0)) continue;
+            Lines gk = k_lines(L, K2);
+            lj.j[nj] = RLoadHPair{L.S[K2].as<float2>(), ZMap{}, gk, L.n[K2], wpair};
+            sj.j[nj] = RStoreRPairBlocks{c, block_map(L, K2), gk.nlines, es};
+            pairs = std::max(pairs, (gk.nlines + 1) / 2);
+            done[K2] = true;
+            ++nj;
+        }
+        FFTLen* f = get_fft(D.ffts, L.n[K]);
+        launch_line<true>(*f, lj, sj, pairs, nj, K != 0, st, "dec_c2r_blocks");
+    }
+}
+
+// The R2C along K of level L's subbands into the hourglasses' spectra; wpair as
+// above (2: the adjoint of the C2R).
+void blocks_r2c(DecPlan& D, DecLevelDev& L, const float* c, int es, float wpair, cudaStream_t st) {
+    bool done[3] = {false, false, false};
+    for (int K = 0; K < 3; ++K) {
+        if (done[K]) continue;
+        LoadJobs<RLoadRPairBlocks> lj{};
+        StoreJobs<RStoreHalfPair> sj{};
+        int nj = 0, pairs = 0;
+        for (int K2 = K; K2 < 3; ++K2) {
+            if (done[K2] || L.n[K2] != L.n[K] || (K2 != 0) != (K != 0)) continue;
+            Lines gk = k_lines(L, K2);
+            lj.j[nj] = RLoadRPairBlocks{c, block_map(L, K2), gk.nlines, es};
+            sj.j[nj] = RStoreHalfPair{L.S[K2].as<float2>(), ZMap{}, gk, L.n[K2], wpair};
+            pairs = std::max(pairs, (gk.nlines + 1) / 2);
+            done[K2] = true;
+            ++nj;
+        }
+        FFTLen* f = get_fft(D.ffts, L.n[K]);
+        launch_line<false>(*f, lj, sj, pairs, nj, K != 0, st, "dec_r2c_blocks");
+    }
 }
 
 // Level j of the analysis after the plane pass (irc_plane_launch_levels<false>,
@@ -1145,25 +1212,7 @@ void scale_forward(DecPlan& D, int j, float* c, int es, cudaStream_t st) {
     }
     // the block FFTs of the other hourglasses, grouped by length and layout
     block_fft_level(D, L, true, fuse, st);
-    // the C2R along K into the subbands: the hourglasses of one length and line layout in one launch
-    bool done[3] = {false, false, false};
-    for (int K = 0; K < 3; ++K) {
-        if (done[K]) continue;
-        LoadJobs<RLoadHPair> lj{};
-        StoreJobs<RStoreRPairBlocks> sj{};
-        int nj = 0, pairs = 0;
-        for (int K2 = K; K2 < 3; ++K2) {
-            if (done[K2] || L.n[K2] != L.n[K] || (K2 != 0) != (K != 0)) continue;
-            Lines gk = k_lines(L, K2);
-            lj.j[nj] = RLoadHPair{L.S[K2].as<float2>(), ZMap{}, gk, L.n[K2]};
-            sj.j[nj] = RStoreRPairBlocks{c, block_map(L, K2), gk.nlines, es};
-            pairs = std::max(pairs, (gk.nlines + 1) / 2);
-            done[K2] = true;
-            ++nj;
-        }
-        FFTLen* f = get_fft(D.ffts, L.n[K]);
-        launch_line<true>(*f, lj, sj, pairs, nj, K != 0, st, "dec_c2r_blocks");
-    }
+    blocks_c2r(D, L, c, es, 1.f, st);
 }
 
 // Level j of the synthesis up to the plane pass (irc_plane_launch_levels<true>,
@@ -1173,25 +1222,7 @@ void scale_forward(DecPlan& D, int j, float* c, int es, cudaStream_t st) {
 // hourglasses' stages.
 void scale_inverse(DecPlan& D, int j, const float* c, int es, cudaStream_t st) {
     DecLevelDev& L = *D.lv[j];
-    // the R2C along K out of the subbands: the hourglasses of one length and line layout in one launch
-    bool done[3] = {false, false, false};
-    for (int K = 0; K < 3; ++K) {
-        if (done[K]) continue;
-        LoadJobs<RLoadRPairBlocks> lj{};
-        StoreJobs<RStoreHalfPair> sj{};
-        int nj = 0, pairs = 0;
-        for (int K2 = K; K2 < 3; ++K2) {
-            if (done[K2] || L.n[K2] != L.n[K] || (K2 != 0) != (K != 0)) continue;
-            Lines gk = k_lines(L, K2);
-            lj.j[nj] = RLoadRPairBlocks{c, block_map(L, K2), gk.nlines, es};
-            sj.j[nj] = RStoreHalfPair{L.S[K2].as<float2>(), ZMap{}, gk, L.n[K2]};
-            pairs = std::max(pairs, (gk.nlines + 1) / 2);
-            done[K2] = true;
-            ++nj;
-        }
-        FFTLen* f = get_fft(D.ffts, L.n[K]);
-        launch_line<false>(*f, lj, sj, pairs, nj, K != 0, st, "dec_r2c_blocks");
-    }
+    blocks_r2c(D, L, c, es, 1.f, st);
     // the block FFTs of the hourglasses whose plane pass does not run them, grouped by length and layout
     bool fuse[3];
     for (int K = 0; K < 3; ++K) fuse[K] = irc_plane_fuses<true>(L, K);
@@ -1253,79 +1284,84 @@ void scale_inverse_sum_merge(DecPlan& D, int j, cudaStream_t st) {
     if (!L.merge_fused) pyr_merge(D, j, st);
 }
 
-// Adjoint of scale_forward: the subbands of level j (real, in c) to the
-// level's spectrum.  Per hourglass: a_k * R2C along K (a_k = 2 off the
-// self-conjugate bins: the adjoint of the C2R), forward block FFTs (adjoint of
-// the backward ones), the IRC stages in reverse order conjugate-transposed;
-// then the zero-padded sum of V_K s_K S_K.
+// Level j of the analysis' transpose up to the plane pass
+// (irc_plane_launch_levels<true> with adjoint): a_k times the R2C along K out
+// of the subbands (a_k = 2 off the self-conjugate bins: the adjoint of the
+// C2R), the forward block FFTs (adjoint of the backward ones) the plane pass
+// does not run, and the stages, in reverse order conjugate-transposed, of the
+// hourglasses whose plane does not fit.
 void scale_forward_adjoint(DecPlan& D, int j, const float* c, int es, cudaStream_t st) {
+    DecLevelDev& L = *D.lv[j];
+    blocks_r2c(D, L, c, es, 2.f, st);
+    bool fuse[3];
+    for (int K = 0; K < 3; ++K) fuse[K] = irc_plane_fuses<true>(L, K);
+    block_fft_level(D, L, false, fuse, st);
+    for (int K = 0; K < 3; ++K) {
+        const int* hd = L.hd[K];
+        if (irc_plane_fits(L, K)) continue;
+        for (int sg_i = (int)L.stages[K].size() - 1; sg_i >= 0; --sg_i) {
+            auto& sg = L.stages[K][sg_i];
+            int tok = prof_begin("dec_irc", st);
+            irc_stage_kernel<<<irc_stage_grid(hd, sg.m), grid3_threads(), 0, st>>>(
+                L.S[K].as<float2>(), hd[0], hd[1], hd[2], K, sg.m, sg.b, sg.f[0].as<float2>(), sg.f[1].as<float2>(), 1, 1);
+            prof_end(tok, st);
+            cuda_check(cudaGetLastError(), "irc_stage_kernel");
+        }
+    }
+}
+
+// Level j of the analysis' transpose after the plane pass: the zero-padded sum
+// of V_K s_K S_K into the level's spectrum, then the adjoint of its split.
+void scale_forward_adjoint_sum(DecPlan& D, int j, cudaStream_t st) {
     DecLevelDev& L = *D.lv[j];
     HermArgs ha;
     float sK[3];
     for (int K = 0; K < 3; ++K) {
-        const int* hd = L.hd[K];
-        float2* S = L.S[K].as<float2>();
-        Lines gk = k_lines(L, K);
-        FFTLen* f = get_fft(D.ffts, L.n[K]);
-        BlockMap bm = block_map(L, K);
-        int pairs = (gk.nlines + 1) / 2;
-        launch_line<false>(*f, RLoadRPairBlocks{c, bm, gk.nlines, es}, RStoreHalfPair{S, ZMap{}, gk, L.n[K], 2.f}, pairs,
-                           1, K != 0, st, "dec_r2c_blocks");
-        for (int m = 0; m < 3; ++m)
-            if (m != K) block_fft(D, S, hd, m, L.bsize[K][m], false, st);
-        for (int sg_i = (int)L.stages[K].size() - 1; sg_i >= 0; --sg_i) {
-            auto& sg = L.stages[K][sg_i];
-            int tok = prof_begin("dec_irc", st);
-            irc_stage_kernel<<<irc_stage_grid(hd, sg.m), grid3_threads(), 0, st>>>(S, hd[0], hd[1], hd[2], K, sg.m, sg.b,
-                                                                sg.f[0].as<float2>(), sg.f[1].as<float2>(), 1, 1);
-            prof_end(tok, st);
-            cuda_check(cudaGetLastError(), "irc_stage_kernel");
-        }
         int sb[3];
         for (int d = 0; d < 3; ++d) sb[d] = d == K ? L.n[K] : L.bsize[K][d];
         sK[K] = (float)(1.0 / ((double)sb[0] * sb[1] * sb[2]));
-        ha.S[K] = S;
+        ha.S[K] = L.S[K].as<float2>();
         ha.V[K] = L.V[K].as<float>();
     }
     int tok = prof_begin("dec_hg_adjoint", st);
-    hg_adjoint_sum_kernel<<<grid3_blocks(L.n[0], L.n[1], L.n[2]), grid3_threads(), 0, st>>>(D.spectra[j]->as<float2>(), L.n[0], L.n[1], L.n[2], ha,
-                                                          sK[0], sK[1], sK[2]);
+    hg_adjoint_sum_kernel<<<grid3_blocks(L.n[0], L.n[1], L.n[2]), grid3_threads(), 0, st>>>(
+        D.spectra[j]->as<float2>(), L.n[0], L.n[1], L.n[2], ha, sK[0], sK[1], sK[2]);
     prof_end(tok, st);
     cuda_check(cudaGetLastError(), "hg_adjoint_sum_kernel");
+    pyr_merge(D, j, st, true);
 }
 
-// Adjoint of scale_inverse: the level's spectrum to its subbands.  Per
-// hourglass: the gather adjoint to the Hermitian sum, the synthesis IRC
-// stages in forward order conjugate-transposed, backward block FFTs, and the
-// C2R along K of S / a_k (the adjoint of the R2C).
+// Level j of the synthesis' transpose after the plane pass
+// (irc_plane_launch_levels<false> with adjoint, which gathers the adjoint of
+// the Hermitian sum on load): the gather and the synthesis stages, in forward
+// order conjugate-transposed, of the hourglasses whose plane does not fit, the
+// backward block FFTs it does not run, and the C2R along K of S / a_k (the
+// adjoint of the R2C).
 void scale_inverse_adjoint(DecPlan& D, int j, float* c, int es, cudaStream_t st) {
     DecLevelDev& L = *D.lv[j];
+    bool fuse[3];
     for (int K = 0; K < 3; ++K) {
         const int* hd = L.hd[K];
         float2* S = L.S[K].as<float2>();
+        fuse[K] = irc_plane_fuses<false>(L, K);
+        if (irc_plane_fits(L, K)) continue;
         {
             int tok = prof_begin("dec_herm_gather", st);
-            herm_gather_kernel<<<grid3_blocks(hd[0], hd[1], hd[2]), grid3_threads(), 0, st>>>(D.spectra[j]->as<float2>(), L.n[0], L.n[1], L.n[2], S,
-                                                               L.V[K].as<float>(), K, 1.0f / 3.0f);
+            herm_gather_kernel<<<grid3_blocks(hd[0], hd[1], hd[2]), grid3_threads(), 0, st>>>(
+                D.spectra[j]->as<float2>(), L.n[0], L.n[1], L.n[2], S, L.V[K].as<float>(), K, 1.0f / 3.0f);
             prof_end(tok, st);
             cuda_check(cudaGetLastError(), "herm_gather_kernel");
         }
         for (auto& sg : L.stages[K]) {
             int tok = prof_begin("dec_irc", st);
-            irc_stage_kernel<<<irc_stage_grid(hd, sg.m), grid3_threads(), 0, st>>>(S, hd[0], hd[1], hd[2], K, sg.m, sg.b,
-                                                                sg.f[2].as<float2>(), sg.f[3].as<float2>(), 0, 1);
+            irc_stage_kernel<<<irc_stage_grid(hd, sg.m), grid3_threads(), 0, st>>>(
+                S, hd[0], hd[1], hd[2], K, sg.m, sg.b, sg.f[2].as<float2>(), sg.f[3].as<float2>(), 0, 1);
             prof_end(tok, st);
             cuda_check(cudaGetLastError(), "irc_stage_kernel");
         }
-        for (int m = 0; m < 3; ++m)
-            if (m != K) block_fft(D, S, hd, m, L.bsize[K][m], true, st);
-        Lines gk = k_lines(L, K);
-        FFTLen* f = get_fft(D.ffts, L.n[K]);
-        BlockMap bm = block_map(L, K);
-        int pairs = (gk.nlines + 1) / 2;
-        launch_line<true>(*f, RLoadHPair{S, ZMap{}, gk, L.n[K], 0.5f}, RStoreRPairBlocks{c, bm, gk.nlines, es}, pairs, 1,
-                          K != 0, st, "dec_c2r_blocks");
     }
+    block_fft_level(D, L, true, fuse, st);
+    blocks_c2r(D, L, c, es, 0.5f, st);
 }
 
 // f(j, stream) for the levels j = 0 .. J-1, level 0 on st and the others on
@@ -1411,12 +1447,15 @@ void dec_adjoint_analyze(DecPlan& D, const void* c, void* x, cudaStream_t st) {
         float* xout = reinterpret_cast<float*>(x) + ch;
         const int* nl = S.pyramid[D.J - 1].nlow;
         const long long M = (long long)nl[0] * nl[1] * nl[2];
-        fft_real_full(D, cin, es, nl, D.spectra[D.J]->as<float2>(), st);
-        cscale(D.spectra[D.J]->as<float2>(), M, (float)(1.0 / (double)M), st);
-        for (int j = D.J - 1; j >= 0; --j) {
-            scale_forward_adjoint(D, j, cin, es, st);
-            pyr_merge(D, j, st, true);
-        }
+        per_level(D, st, [&](int j, cudaStream_t s) {
+            if (j == D.J - 1) {
+                fft_real_full(D, cin, es, nl, D.spectra[D.J]->as<float2>(), s);
+                cscale(D.spectra[D.J]->as<float2>(), M, (float)(1.0 / (double)M), s);
+            }
+            scale_forward_adjoint(D, j, cin, es, s);
+        });
+        irc_plane_launch_levels<true>(D, st, true);
+        for (int j = D.J - 1; j >= 0; --j) scale_forward_adjoint_sum(D, j, st);
         ifft_full_real(D, D.spectra[0]->as<float2>(), D.dims, xout, es, 1.0f, st);
     }
 }
@@ -1433,12 +1472,14 @@ void dec_adjoint_synthesize(DecPlan& D, const void* x, void* c, cudaStream_t st)
         const long long N = (long long)D.dims[0] * D.dims[1] * D.dims[2];
         fft_real_full(D, xin, es, D.dims, D.spectra[0]->as<float2>(), st);
         cscale(D.spectra[0]->as<float2>(), N, (float)(1.0 / (double)N), st);
-        for (int j = 0; j < D.J; ++j) {
-            pyr_split(D, j, st, true);
-            scale_inverse_adjoint(D, j, cout, es, st);
-        }
+        // as in dec_analyze: every split first, one plane pass, then the levels concurrently
+        for (int j = 0; j < D.J; ++j) pyr_split(D, j, st, true);
+        irc_plane_launch_levels<false>(D, st, true);
         const int* nl = S.pyramid[D.J - 1].nlow;
-        ifft_full_real(D, D.spectra[D.J]->as<float2>(), nl, cout, es, 1.0f, st);
+        per_level(D, st, [&](int j, cudaStream_t s) {
+            scale_inverse_adjoint(D, j, cout, es, s);
+            if (j == D.J - 1) ifft_full_real(D, D.spectra[D.J]->as<float2>(), nl, cout, es, 1.0f, s);
+        });
     }
 }
 
