@@ -68,21 +68,33 @@ struct AnyGeom : AnyLine<N> {
     static constexpr int THREADS = LP * AnyLine<N>::N2;
     static constexpr int XROW = AnyLine<N>::N2 + 1;              // exchange row pitch (float2)
     static constexpr int XLINE = (AnyLine<N>::N1 * XROW) | 1;    // exchange line pitch, odd
-    static constexpr size_t SMEM = sizeof(float2) * (size_t)LP * XLINE;
+    static constexpr size_t SMEM = sizeof(float2) * ((size_t)N + (size_t)LP * XLINE);   // twiddles, exchange rows
 };
+
+// Twiddles of a line FFT rearranged as tw2[m N2 + p] = w_N^{p m}.
+template <int N>
+__device__ __forceinline__ void any_load_twiddles(float2* tw2, const float2* __restrict__ tw) {
+    using L = AnyLine<N>;
+    for (int i = threadIdx.x; i < N; i += blockDim.x) {
+        const int m = i / L::N2, p = i - m * L::N2;
+        tw2[i] = tw[p * m];
+    }
+}
 
 // The FFT of one line of a block pass from values in registers: v[r] =
 // x[p + N2 r]; u as AnyLine says.  One barrier; the exchange rows may be
-// rewritten after the next one.
+// rewritten after the next one.  The twiddles tw2 lie in shared memory: read from
+// global memory they are loop constants to the compiler, which then holds them
+// in registers across the terms and spills.
 template <int N, bool INV>
-__device__ __forceinline__ void any_block_fft(float2 (&v)[AnyLine<N>::N1], int p, float2* xl,
-                                              const float2* __restrict__ tw, float2 (&u)[AnyLine<N>::E]) {
+__device__ __forceinline__ void any_block_fft(float2 (&v)[AnyLine<N>::N1], int p, float2* xl, const float2* tw2,
+                                              float2 (&u)[AnyLine<N>::E]) {
     using G = AnyGeom<N>;
     constexpr int N1 = G::N1, N2 = G::N2;
     RegDft<N1, INV>::run(v);
 #pragma unroll
     for (int m = 1; m < N1; ++m) {
-        float2 w = __ldg(&tw[p * m]);
+        float2 w = tw2[m * N2 + p];
         if (INV) w.y = -w.y;
         v[m] = c_mul(v[m], w);
     }
@@ -109,16 +121,6 @@ template <int N>
 __device__ __forceinline__ int any_pair_line(int s) {
     if (AnyLine<N>::N2 == 8) return s == 1 ? 2 : (s == 2 ? 1 : s);
     return s;
-}
-
-// Twiddles of a warp line FFT rearranged as tw2[m N2 + p] = w_N^{p m}.
-template <int N>
-__device__ __forceinline__ void any_load_twiddles(float2* tw2, const float2* __restrict__ tw) {
-    using L = AnyLine<N>;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        const int m = i / L::N2, p = i - m * L::N2;
-        tw2[i] = tw[p * m];
-    }
 }
 
 // FFT of one line by the N2 lanes p of a warp, exchanged through N slots of

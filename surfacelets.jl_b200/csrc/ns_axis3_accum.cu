@@ -7,12 +7,20 @@ namespace sfl {
 
 namespace {
 
+// Resident CTAs an SM the register budget aims at: three (85 registers a
+// thread) where a thread holds nine or ten values and sums, two (128) else.
+// The pass waits on L2 and gains from more warps (120 x 100 x 90 synthesis 297
+// -> 258 us), and loses far more to spilled registers (three CTAs at 128 points:
+// 489 -> 534 us).
+template <int N>
+constexpr int accum_minb() { return AnyLine<N>::N1 <= 10 && AnyLine<N>::E > 8 && AnyLine<N>::E <= 10 ? 3 : 2; }
 // Lengths whose sums go to shared memory (their register form spills).
 template <int N>
 constexpr bool accum_sums_shared() { return AnyLine<N>::E > 8; }
 template <int N>
 constexpr size_t accum_smem() {
-    return AnyGeom<N>::SMEM + (accum_sums_shared<N>() ? sizeof(float2) * AnyLine<N>::E * AnyGeom<N>::THREADS : 0);
+    return AnyGeom<N>::SMEM +
+           (accum_sums_shared<N>() ? (sizeof(float2) + sizeof(float)) * AnyLine<N>::E * AnyGeom<N>::THREADS : 0);
 }
 
 // Synthesis line pass over a chunk's segments: per segment FFT_3 of every item
@@ -31,14 +39,18 @@ constexpr size_t accum_smem() {
 // nbq plane-b wedges q times whole rows p (item t = p nbq + q); otherwise
 // every item is its own term.  Terms are added in q order.
 template <int N>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, accum_minb<N>())
     ns_slab_accum_kernel(const float2* __restrict__ Y, long long ystride, int P1, int s3, BoxMap un,
                          const __grid_constant__ NSMaskTables tb, const __grid_constant__ Chunk ck, int synth,
                          float2* acc, float2* comp, const float2* __restrict__ tw, long long ychs, long long achs,
                          long long agrp) {
     using Ge = AnyGeom<N>;
     constexpr int N1 = Ge::N1, N2 = Ge::N2, LP = Ge::LP, E = Ge::E;
-    extern __shared__ float2 xch[];
+    extern __shared__ float2 a3_sm[];
+    float2* const tws = a3_sm;
+    float2* const xch = a3_sm + N;
+    any_load_twiddles<N>(tws, tw);
+    __syncthreads();
     Y += blockIdx.y * ychs;   // channel
     acc += blockIdx.y * achs + blockIdx.z * agrp;
     comp += blockIdx.y * achs + blockIdx.z * agrp;
@@ -60,6 +72,15 @@ __global__ void __launch_bounds__(256, 2)
         else
             return sr[q];
     };
+    // the line's group factors, in registers or beside the sums
+    float gr[kSumsShared ? 1 : E];
+    float* gs = reinterpret_cast<float*>(xch + LP * Ge::XLINE + (kSumsShared ? E * Ge::THREADS : 0)) + tid;
+    auto gf = [&](int q) -> float& {
+        if constexpr (kSumsShared)
+            return gs[q * Ge::THREADS];
+        else
+            return gr[q];
+    };
     const int si = tb.h1 * tb.n2;
     const bool wedge_masks = !(synth && !tb.tight);
     const float2* yl = Y + k1 + P1 * k2;
@@ -73,7 +94,6 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
         for (int q = 0; q < E; ++q) sum(q) = make_float2(0.f, 0.f);
         // the group factor of the line (group table, bandpass table or the lowpass factors), once for all items
-        float gf[E];
         {
             const NSMaskLine m0 = chunk_mask_line(tb, sg, ck.item[sg.i0], k1, k2, synth != 0);
 #pragma unroll
@@ -81,7 +101,7 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
                 for (int k = 0; k < N2; ++k) {
                     const int k3 = Ge::has(p, j) ? (p + N2 * j) + N1 * k : 0;
-                    gf[j * N2 + k] = m0.low ? m0.lowc * m0.lowv[k3] : m0.m[(long long)k3 * si];
+                    gf(j * N2 + k) = m0.low ? m0.lowc * m0.lowv[k3] : m0.m[k3 * si];
                 }
         }
         const int nbq = sg.nbq;
@@ -92,64 +112,52 @@ __global__ void __launch_bounds__(256, 2)
             const ChunkItem& it0 = ck.item[sg.i0 + t];
             const bool before = wedge_masks && !sg.low && it0.wa_hi != 2;   // plane a applied before the FFT
             // the term: sum_p wa_p Y_pq (one item with weight 1 when plane a varies along the line; x 1 is
-            // exact).  The loads of the next item are in flight while the current one is added.
+            // exact).
             const int nt = before ? rows : 1;
             auto weight = [&](int z) {
                 const ChunkItem& it = ck.item[z];
                 return before ? __ldg(tb.planes + it.wa_off + (it.wa_lo == 0 ? k1 : k2) + it.wa_dlo * k2) : 1.f;
             };
+            // opaque to the compiler, which would otherwise keep the lines' offsets of all loops in registers and
+            // spill others for them (176 bytes a thread at 128 points)
+            int s3t = s3, wst = 1;
+            asm volatile("" : "+r"(s3t), "+r"(wst));
             float2 v[N1], yb[N1];
             const int z0 = sg.i0 + t;
             float wz = weight(z0);
             {
                 const float2* yz = yl + z0 * ystride;
 #pragma unroll
-                for (int r = 0; r < N1; ++r) yb[r] = valid ? yz[(long long)(p + N2 * r) * s3] : make_float2(0.f, 0.f);
+                for (int r = 0; r < N1; ++r) yb[r] = valid ? yz[(p + N2 * r) * s3t] : make_float2(0.f, 0.f);
             }
 #pragma unroll 1
             for (int pp = 0; pp < nt; ++pp) {
                 const float az = wz;
-                if constexpr (N1 <= 16) {
-                    // a second buffer for the next item's loads (long lines would spill it)
-                    float2 cur[N1];
 #pragma unroll
-                    for (int r = 0; r < N1; ++r) cur[r] = yb[r];
-                    if (pp + 1 < nt) {
-                        const int z = z0 + (pp + 1) * nbq;
-                        const float2* yz = yl + z * ystride;
-                        wz = weight(z);
+                for (int r = 0; r < N1; ++r) v[r] = pp == 0 ? c_scale(yb[r], az) : c_fma(yb[r], az, v[r]);
+                if (pp + 1 < nt) {
+                    const int z = z0 + (pp + 1) * nbq;
+                    const float2* yz = yl + z * ystride;
+                    wz = weight(z);
 #pragma unroll
-                        for (int r = 0; r < N1; ++r)
-                            yb[r] = valid ? yz[(long long)(p + N2 * r) * s3] : make_float2(0.f, 0.f);
-                    }
-#pragma unroll
-                    for (int r = 0; r < N1; ++r) v[r] = pp == 0 ? c_scale(cur[r], az) : c_fma(cur[r], az, v[r]);
-                } else {
-#pragma unroll
-                    for (int r = 0; r < N1; ++r) v[r] = pp == 0 ? c_scale(yb[r], az) : c_fma(yb[r], az, v[r]);
-                    if (pp + 1 < nt) {
-                        const int z = z0 + (pp + 1) * nbq;
-                        const float2* yz = yl + z * ystride;
-                        wz = weight(z);
-#pragma unroll
-                        for (int r = 0; r < N1; ++r)
-                            yb[r] = valid ? yz[(long long)(p + N2 * r) * s3] : make_float2(0.f, 0.f);
-                    }
+                    for (int r = 0; r < N1; ++r)
+                        yb[r] = valid ? yz[(p + N2 * r) * s3t] : make_float2(0.f, 0.f);
                 }
             }
             float2 u[E];
             if (t > 0) __syncthreads();   // the exchange rows were read for the previous term
-            any_block_fft<N, false>(v, p, xl, tw, u);
+            any_block_fft<N, false>(v, p, xl, tws, u);
             // the term's first item carries plane b and the group factor
             const NSMaskLine mk = chunk_mask_line(tb, sg, it0, k1, k2, synth != 0);
             const bool wedges = !(mk.low || mk.plain);
+            const int was = mk.was * wst, wbs = mk.wbs * wst;
 #pragma unroll
             for (int j = 0; j < Ge::M; ++j)
 #pragma unroll
                 for (int k = 0; k < N2; ++k) {
                     const int k3 = Ge::has(p, j) ? (p + N2 * j) + N1 * k : 0;
-                    const float g = gf[j * N2 + k];
-                    const float m = !wedges ? g : (before ? g * mk.wb[k3 * mk.wbs] : g * (mk.wa[k3 * mk.was] * mk.wb[k3 * mk.wbs]));
+                    const float g = gf(j * N2 + k);
+                    const float m = !wedges ? g : (before ? g * mk.wb[k3 * wbs] : g * (mk.wa[k3 * was] * mk.wb[k3 * wbs]));
                     float2& tsum = sum(j * N2 + k);
                     tsum = make_float2(fmaf(u[j * N2 + k].x, m, tsum.x), fmaf(u[j * N2 + k].y, m, tsum.y));
                 }
@@ -157,10 +165,11 @@ __global__ void __launch_bounds__(256, 2)
         if (valid) {
             float2* a = acc + k1 + P1 * k2;
             float2* ca = comp + k1 + P1 * k2;
-#pragma unroll
+            // four bins at a time: all of them at once spill
+#pragma unroll(kSumsShared ? 1 : Ge::M)
             for (int j = 0; j < Ge::M; ++j)
                 if (Ge::has(p, j)) {
-#pragma unroll
+#pragma unroll(kSumsShared ? 4 : N2)
                     for (int k = 0; k < N2; ++k) {
                         const int o = ((p + N2 * j) + N1 * k) * s3;
                         float2 sv = a[o], cv = ca[o];

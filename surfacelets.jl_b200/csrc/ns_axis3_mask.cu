@@ -28,7 +28,11 @@ __global__ void __launch_bounds__(256, 2)
                               long long ychs) {
     using Ge = AnyGeom<N>;
     constexpr int N1 = Ge::N1, N2 = Ge::N2, LP = Ge::LP, E = Ge::E;
-    extern __shared__ float2 xch[];
+    extern __shared__ float2 a3_sm[];
+    float2* const tws = a3_sm;
+    float2* const xch = a3_sm + N;
+    any_load_twiddles<N>(tws, tw);
+    __syncthreads();
     X += blockIdx.y * xchs;   // channel
     Y += blockIdx.y * ychs;
     const int t = mask_tile_of(tl, blockIdx.x);
@@ -52,8 +56,8 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
         for (int r = 0; r < N1; ++r) {
             const int i = p + N2 * r;
-            const float g = m0.low ? m0.lowc * m0.lowv[i] : m0.m[(long long)i * si];
-            xg[r] = valid ? c_scale(xp[(long long)i * s3], g) : make_float2(0.f, 0.f);
+            const float g = m0.low ? m0.lowc * m0.lowv[i] : m0.m[i * si];
+            xg[r] = valid ? c_scale(xp[i * s3], g) : make_float2(0.f, 0.f);
         }
     }
     float2 u[E];
@@ -85,7 +89,7 @@ __global__ void __launch_bounds__(256, 2)
                 }
             }
             if (k > k0) __syncthreads();   // the exchange rows were read for the previous FFT
-            any_block_fft<N, true>(v, p, xl, tw, u);
+            any_block_fft<N, true>(v, p, xl, tws, u);
         }
         if (valid) {
             const float a0 = after ? mk.wa[0] : 1.f;

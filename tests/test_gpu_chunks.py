@@ -35,3 +35,19 @@ def test_chunks_do_not_change_results(sfl, dims, levels, dtype):
     assert torch.equal(sfl.adjoint_synthesize(a, x), sfl.adjoint_synthesize(b, x))
     if dtype == "float32":
         assert torch.equal(sfl.denoise(a, x, 0.3), sfl.denoise(b, x, 0.3))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(16, 18, 20), (17, 19, 21), (32, 32, 32)])
+def test_bf16_packing_is_the_float_subbands_rounded(sfl, dims):
+    """Four values a step (volumes of a multiple of four) and one: exact, since
+    packing rounds the float32 subband by its power-of-two scale once."""
+    x = sfl.to_device(np.random.default_rng(4).standard_normal(dims).astype(np.float32))
+    ws = sfl.make_workspace(sfl.NSSurfacelet(direction_levels=[1, 2], bernstein_order=6), "float32", dims)
+    c = sfl.analyze(ws, x)
+    q, scales = sfl.analyze_bf16(ws, x)
+    peak = c.abs().amax((0, 1, 2))
+    assert torch.equal(scales, torch.ldexp(torch.ones_like(peak), torch.frexp(peak)[1]))
+    assert torch.equal(q, (c / scales).to(torch.bfloat16))
+    y = sfl.synthesize_bf16(ws, q, scales)
+    assert torch.equal(y, sfl.synthesize(ws, sfl.as_colmajor(q.float() * scales)))
