@@ -410,10 +410,11 @@ void ns_plan_init(NSPlan& P, const sfl_ns_params& p, const int dims[3], int dtyp
 void ns_alloc_scratch(NSPlan& P) {
     const long long spec = P.slab ? P.SP : P.H;
     P.X.alloc(sizeof(float2) * spec * P.nch);
-    P.slots = P.slab ? ns_slab_slots(P) : P.group;
+    P.slots = P.group;
+    if (P.slab) ns_slab_slots(P);
     P.work.alloc(sizeof(float2) * spec * P.slots * (P.slab ? P.nch : 1));
     P.ngrp = P.slab ? ns_slab_groups(P) : 1;
-    P.rcomp.alloc(P.ngrp > 1 ? sizeof(float2) * spec * P.nch : 0);
+    P.rcomp = DevMem();   // allocated by the first item-range accumulation
     if (P.slab) {
         P.acc.alloc(sizeof(float2) * spec * P.nch * P.ngrp);
         P.comp.alloc(sizeof(float2) * spec * P.nch * P.ngrp);
@@ -660,6 +661,7 @@ void ns_acc_clear(NSPlan& P, float2* acc, float2* comp, cudaStream_t st) {
 }
 
 float2* ns_range_comp(NSPlan& P, int ch) {
+    if (P.ngrp > 1 && !P.rcomp.p) P.rcomp.alloc(sizeof(float2) * ns_spec_elems(P) * P.nch);
     return (P.ngrp > 1 ? P.rcomp : P.comp).as<float2>() + ch * ns_spec_elems(P);
 }
 

@@ -449,9 +449,15 @@ void launch_any_slab_es(const NSPlan& P, const SlabArgs& a, cudaStream_t st, con
     const int n1 = P.dims[0], n2 = P.dims[1];
     const size_t smem = any_smem(n1, n2, a.P1);
     const int threads = 32 * any_warps(n1, n2, smem);
-    int resident = 0;
-    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, threads, smem),
-               "cudaOccupancyMaxActiveBlocksPerMultiprocessor(any slab)");
+    // the last geometry's answer: the query costs as much as a launch
+    thread_local int resident = 0, asked_threads = -1;
+    thread_local size_t asked_smem = 0;
+    if (asked_threads != threads || asked_smem != smem) {
+        cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, threads, smem),
+                   "cudaOccupancyMaxActiveBlocksPerMultiprocessor(any slab)");
+        asked_threads = threads;
+        asked_smem = smem;
+    }
     const int grid = std::max(1, std::min(a.units, std::max(resident, 1) * P.sms));
     int tok = prof_begin(tag, st);
     kern<<<grid, threads, smem, st>>>(a, n1, n2);

@@ -277,9 +277,15 @@ void launch_mix_slab_b(const SlabArgs& a, const MixSlabGeom& g, int sms, cudaStr
     const size_t smem = mix_slab_smem(g, a.P1, KIND);
     const int items = std::max(mix_items(g.a1.sc), mix_items(g.a2.sc)) << g.lg;
     const int threads = std::min(kMixSlabThreads, std::max(64, (items + 31) / 32 * 32));
-    int resident = 0;
-    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, threads, smem),
-               "cudaOccupancyMaxActiveBlocksPerMultiprocessor(mix slab)");
+    // the last geometry's answer: the query costs as much as a launch
+    thread_local int resident = 0, asked_threads = -1;
+    thread_local size_t asked_smem = 0;
+    if (asked_threads != threads || asked_smem != smem) {
+        cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, threads, smem),
+                   "cudaOccupancyMaxActiveBlocksPerMultiprocessor(mix slab)");
+        asked_threads = threads;
+        asked_smem = smem;
+    }
     const int grid = std::max(1, std::min(a.units, std::max(resident, 1) * sms));
     int tok = prof_begin(tag, st);
     kern<<<grid, threads, smem, st>>>(a, g);

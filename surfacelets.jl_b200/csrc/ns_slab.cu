@@ -236,7 +236,6 @@ Chunk make_chunk(const NSPlan& P, int i0, int nz, bool synth_masks) {
             ci.nk1 = sg.nk1;
             ci.nk2 = sg.nk2;
             ci.b2 = sg.b2;
-            ci.seg = (short)c.nseg;
         }
         ++c.nseg;
         a = e;
@@ -552,10 +551,18 @@ NSBox ns_table_box(const std::vector<double>& g, int h1, int n2, int n3) {
 // Work slots of the slab pipeline: the group when one was chosen, else as many
 // spectra as 256 MB hold (complex volumes: two channels each), so that a chunk
 // spans the mask groups of small boxes.
-int ns_slab_slots(const NSPlan& P) {
-    if (P.group != std::min(8, P.S)) return P.group;
+// No more than the transforms' own chunks use.
+void ns_slab_slots(NSPlan& P) {
+    P.slots = P.group;
+    if (P.group != std::min(8, P.S)) return;
     const long long fit = (256LL << 20) / (8 * P.SP * P.nch);
-    return (int)std::max<long long>(P.group, std::min<long long>({fit, (long long)kChunkItems, (long long)P.S}));
+    P.slots = (int)std::max<long long>(P.group, std::min<long long>({fit, (long long)kChunkItems, (long long)P.S}));
+    int used = P.group;
+    for (int i0 = 0, i1; i0 < P.S; i0 = i1) {
+        i1 = chunk_end(P, i0);
+        used = std::max(used, i1 - i0);
+    }
+    P.slots = used;
 }
 
 NSBox ns_make_box(int nk1, int b2, int n2) {

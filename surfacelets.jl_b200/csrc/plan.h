@@ -202,7 +202,7 @@ void ns_slab_acc_clear(NSPlan& P, float2* acc, float2* comp, cudaStream_t st);
 // The plan's accumulators of channel ch added into a caller's spectrum A with compensation C.
 void ns_merge_groups(NSPlan& P, int ch, float2* A, float2* C, cudaStream_t st);
 float2* ns_range_comp(NSPlan& P, int ch);
-int ns_slab_slots(const NSPlan& P);
+void ns_slab_slots(NSPlan& P);
 NSBox ns_make_box(int nk1, int b2, int n2);
 NSBox ns_table_box(const std::vector<double>& g, int h1, int n2, int n3);
 void ns_alloc_scratch(NSPlan& P);
