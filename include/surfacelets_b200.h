@@ -185,7 +185,9 @@ int sfl_plan_status(sfl_plan* plan, int32_t* status, int32_t reset);
 int sfl_plan_selftest_wait(sfl_plan* plan, void* stream);
 
 /* Subbands a launch keeps in flight (NS: scratch holds that many spectra).
- * Default 8; only affects speed and scratch size. */
+ * Default 8, of one mask group; left at the default, the slab pipelines put
+ * several mask groups in a launch and hold as many spectra as those take, up
+ * to 256 MB.  Only affects speed and scratch size. */
 int sfl_plan_set_group(sfl_plan* plan, int32_t group);
 
 /* NSSurfacelet kernel pipeline.  All give the same subbands to float32
