@@ -337,7 +337,9 @@ int sfl_ns_denoise(sfl_plan* plan, const void* x, void* y, const float* tau, voi
  *   analyze_range      the subbands at positions [first, first + count) from
  *                      X into count consecutive volumes of c;
  *   accumulate_range   their synthesis contributions into the spectrum A
- *                      (clear != 0 zeroes A first);
+ *                      (clear != 0 zeroes A first; clear == 0 adds to what A
+ *                      holds, from the first call on a plan too, and carries
+ *                      on the plan's rounding compensation);
  *   inverse_spectrum   x from an accumulated spectrum (A is overwritten).
  * Accumulated spectra add: the sum over devices of each device's
  * accumulation of its own ranges is the accumulation of all of them.  Slab

@@ -1103,7 +1103,7 @@ int sfl_ns_accumulate_range(sfl_plan* plan, const void* c, int32_t first, int32_
                 float2* comp = sfl::ns_range_comp(N, ch);
                 if (clear) sfl::ns_acc_clear(N, acc, comp, as_stream(stream));
                 // with several accumulators the range goes through the plan's, then into A
-                const bool groups = N.slab && N.ngrp > 1;
+                const bool groups = N.slab && N.ngrp > 1 && count > 0;
                 float2* to = groups ? N.acc.as<float2>() + ch * E : acc;
                 float2* tc = groups ? sfl::ns_comp_grid(N, ch) : comp;
                 if (groups) sfl::ns_acc_clear(N, to, tc, as_stream(stream));

@@ -414,14 +414,18 @@ void ns_alloc_scratch(NSPlan& P) {
     if (P.slab) ns_slab_slots(P);
     P.work.alloc(sizeof(float2) * spec * P.slots * (P.slab ? P.nch : 1));
     P.ngrp = P.slab ? ns_slab_groups(P) : 1;
-    P.rcomp = DevMem();   // allocated by the first item-range accumulation
     if (P.slab) {
         P.acc.alloc(sizeof(float2) * spec * P.nch * P.ngrp);
-        P.comp.alloc(sizeof(float2) * spec * P.nch * P.ngrp);
+        // with several accumulators, then the compensation of a caller's spectrum (ns_range_comp)
+        P.comp.alloc(sizeof(float2) * spec * P.nch * (P.ngrp + (P.ngrp > 1 ? 1 : 0)));
     } else {
         P.acc.alloc(sizeof(float2) * P.H * std::max(P.nch, P.group * P.nch));
         P.comp.alloc(sizeof(float2) * P.H * P.nch);
     }
+    // an item range may add to a spectrum that no call on this plan has cleared: its compensation starts at
+    // zero, in place before the caller's streams run (they need not wait for the legacy stream)
+    cuda_check(cudaMemsetAsync(P.comp.p, 0, P.comp.bytes, nullptr), "cudaMemsetAsync(comp)");
+    cuda_check(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
 }
 
 // ── passes ───────────────────────────────────────────────────────────────────
@@ -661,8 +665,8 @@ void ns_acc_clear(NSPlan& P, float2* acc, float2* comp, cudaStream_t st) {
 }
 
 float2* ns_range_comp(NSPlan& P, int ch) {
-    if (P.ngrp > 1 && !P.rcomp.p) P.rcomp.alloc(sizeof(float2) * ns_spec_elems(P) * P.nch);
-    return (P.ngrp > 1 ? P.rcomp : P.comp).as<float2>() + ch * ns_spec_elems(P);
+    const long long E = ns_spec_elems(P);
+    return P.comp.as<float2>() + (P.ngrp > 1 ? P.ngrp * P.nch * E : 0) + ch * E;
 }
 
 float2* ns_comp_grid(NSPlan& P, int ch) { return P.comp.as<float2>() + ch * ns_spec_elems(P); }

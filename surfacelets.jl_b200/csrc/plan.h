@@ -148,8 +148,7 @@ struct NSPlan {
     std::map<int, std::unique_ptr<FFTLen>> ffts;
     DevMem X;        // nch spectra
     DevMem work;     // group spectra
-    DevMem acc, comp;   // ngrp nch accumulators (+ Kahan compensation)
-    DevMem rcomp;       // compensation of a caller's spectrum (item ranges), with several accumulators
+    DevMem acc, comp;   // ngrp nch accumulators; their Kahan compensations, and a caller's spectrum's (item ranges)
     DevMem band, maxbits;   // float32 subbands of a chunk and their peaks (bfloat16 coefficients)
     // streaming state
     int stream_mode = 0;    // 0 idle, 1 analyzing, 2 synthesizing
@@ -201,6 +200,7 @@ int ns_slab_groups(const NSPlan& P);
 void ns_slab_acc_clear(NSPlan& P, float2* acc, float2* comp, cudaStream_t st);
 // The plan's accumulators of channel ch added into a caller's spectrum A with compensation C.
 void ns_merge_groups(NSPlan& P, int ch, float2* A, float2* C, cudaStream_t st);
+// Compensation of a caller's spectrum: the plan's own grid, or with several accumulators one beside theirs.
 float2* ns_range_comp(NSPlan& P, int ch);
 void ns_slab_slots(NSPlan& P);
 NSBox ns_make_box(int nk1, int b2, int n2);
