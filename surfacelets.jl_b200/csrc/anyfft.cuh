@@ -114,19 +114,35 @@ __device__ __forceinline__ void any_block_fft(float2 (&v)[AnyLine<N>::N1], int p
     }
 }
 
-// Lane layout of column pairs (lines 2 P1 slots apart, P1 = 2 mod 4): with four
+// The line that a lane works on.  Lanes without one repeat the warp's first
+// line and drop the values: they read its slots with the lanes it belongs to,
+// between the same warp barriers, and never those of another warp's line,
+// which may be rewritten meanwhile.
+struct LaneLine {
+    int l;
+    bool valid;
+};
+
+// Lane group s = lane / N2 of the warp whose lines start at l0 < nlines.
+template <int N>
+__host__ __device__ __forceinline__ LaneLine any_lane_line(int l0, int s, int nlines) {
+    const bool valid = s < AnyLine<N>::LPW && l0 + s < nlines;
+    return LaneLine{valid ? l0 + s : l0, valid};
+}
+
+// The same for column pairs (lines 2 P1 slots apart, P1 = 2 mod 4): with four
 // lines a warp the two lines of a half warp are two apart, so that their slots
 // fall on disjoint banks.
 template <int N>
-__device__ __forceinline__ int any_pair_line(int s) {
-    if (AnyLine<N>::N2 == 8) return s == 1 ? 2 : (s == 2 ? 1 : s);
-    return s;
+__host__ __device__ __forceinline__ LaneLine any_lane_pair(int l0, int s, int npairs) {
+    return any_lane_line<N>(l0, AnyLine<N>::N2 == 8 && (s == 1 || s == 2) ? 3 - s : s, npairs);
 }
 
 // FFT of one line by the N2 lanes p of a warp, exchanged through N slots of
 // the line's own, base[stride t]: sender q's value m sits at t = N2 m + (q
 // turned by m within N2), which spreads both sides over the banks.  Lanes
-// without a line (valid false) skip the slots but keep to the warp barriers.
+// without a line (valid false) have the slots of one of the warp's lines: they
+// write none and keep to the warp barriers.
 template <int N, bool INV>
 __device__ __forceinline__ void any_warp_fft(float2 (&v)[AnyLine<N>::N1], int p, bool valid,
                                              const float2* __restrict__ tw2, float2* base, int stride,
@@ -154,7 +170,7 @@ __device__ __forceinline__ void any_warp_fft(float2 (&v)[AnyLine<N>::N1], int p,
 #pragma unroll
     for (int j = 0; j < L::M; ++j) {
         float2 w[N2];
-        // lanes without a line or an output read the first slots and are dropped by the caller
+        // lanes without an output read the line's first slots and are dropped by the caller
         const float2* rj = L::has(p, j) ? rb + stride * N2 * N2 * j : base;
 #pragma unroll
         for (int q = 0; q < N2; ++q) w[q] = rj[xo[q]];

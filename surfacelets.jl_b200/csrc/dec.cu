@@ -302,9 +302,7 @@ __device__ __forceinline__ void irc_plane_seg_fft(int ap, int a1, int a2, bool a
     const int nl = (along1 ? a2 : a1) * nseg;
 #pragma unroll 1
     for (int b0 = warp * LN::LPW; b0 < nl; b0 += nwarps * LN::LPW) {
-        const int line = b0 + sl;
-        const bool valid = sl < LN::LPW && line < nl;
-        const int li = valid ? line : 0;
+        const auto [li, valid] = any_lane_line<N>(b0, sl, nl);
         float2* base;
         int stride;
         if (along1) {

@@ -36,9 +36,8 @@ __device__ __noinline__ void any_rows(int so, int P1, int rows, int b2, int k2hi
     const int s = lane / N2, p = lane - s * N2;
 #pragma unroll 1
     for (int l0 = warp * L::LPW; l0 < rows; l0 += step) {
-        const int k1 = l0 + s;
-        const bool valid = s < L::LPW && k1 < rows;
-        float2* row = S + (valid ? k1 : 0);
+        const auto [k1, valid] = any_lane_line<N>(l0, s, rows);
+        float2* row = S + k1;
         float2 v[N1], u[L::E];
         if (!INV || b2 >= N) {
 #pragma unroll
@@ -126,9 +125,9 @@ __device__ __noinline__ void any_cols_inv(int so, int P1, int nk1, int n2, int t
     const int s = lane / N2, p = lane - s * N2, npairs = (n2 + 1) / 2;
 #pragma unroll 1
     for (int l0 = warp * L::LPW; l0 < npairs; l0 += step) {
-        const int l = l0 + any_pair_line<N>(s);
-        const bool valid = s < L::LPW && l < npairs, two = valid && 2 * l + 1 < n2;
-        float2* ca = S + P1 * (2 * (valid ? l : 0));
+        const auto [l, valid] = any_lane_pair<N>(l0, s, npairs);
+        const bool two = valid && 2 * l + 1 < n2;
+        float2* ca = S + P1 * (2 * l);
         float2 v[N1], u[L::E];
         any_load_pair<N>(v, ca, two ? ca + P1 : any_zero(so, P1, n2), nk1, p);
         any_warp_fft<N, true>(v, p, valid, tw2, ca, 1, u);
@@ -142,7 +141,7 @@ __device__ __noinline__ void any_cols_inv(int so, int P1, int nk1, int n2, int t
                 bulk_load(S + P1 * k2, nx.src + P1 * k2, nx.bytes, bar);
             }
         }
-        float* oa = out + ((2 * (valid ? l : 0)) * N + p) * ES;
+        float* oa = out + (2 * l * N + p) * ES;
         float* ob = oa + N * ES;
 #pragma unroll
         for (int j = 0; j < L::M; ++j)
@@ -197,9 +196,9 @@ __device__ __noinline__ void any_cols_fwd(int so, int P1, int nk1, int n2, int t
     const int s = lane / N2, p = lane - s * N2, npairs = (n2 + 1) / 2;
 #pragma unroll 1
     for (int l0 = warp * L::LPW; l0 < npairs; l0 += step) {
-        const int l = l0 + any_pair_line<N>(s);
-        const bool valid = s < L::LPW && l < npairs, two = valid && 2 * l + 1 < n2;
-        const float* ia = in + ((2 * (valid ? l : 0)) * N + p) * ES;
+        const auto [l, valid] = any_lane_pair<N>(l0, s, npairs);
+        const bool two = valid && 2 * l + 1 < n2;
+        const float* ia = in + (2 * l * N + p) * ES;
         const float* ib = ia + (two ? N * ES : 0);
         float2 v[N1], u[L::E];
 #pragma unroll
@@ -208,7 +207,7 @@ __device__ __noinline__ void any_cols_fwd(int so, int P1, int nk1, int n2, int t
 #pragma unroll
             for (int r = 0; r < N1; ++r) v[r].y = 0.f;
         }
-        float2* ca = S + P1 * (2 * (valid ? l : 0));
+        float2* ca = S + P1 * (2 * l);
         any_warp_fft<N, false>(v, p, valid, tw2, ca, 1, u);
         any_put_natural<N>(u, ca, p, valid);
         __syncwarp();
@@ -228,9 +227,9 @@ __device__ __noinline__ void any_cols_shrink(int so, int P1, int nk1, int n2, in
     const int s = lane / N2, p = lane - s * N2, npairs = (n2 + 1) / 2;
 #pragma unroll 1
     for (int l0 = warp * L::LPW; l0 < npairs; l0 += step) {
-        const int l = l0 + any_pair_line<N>(s);
-        const bool valid = s < L::LPW && l < npairs, two = valid && 2 * l + 1 < n2;
-        float2* ca = S + P1 * (2 * (valid ? l : 0));
+        const auto [l, valid] = any_lane_pair<N>(l0, s, npairs);
+        const bool two = valid && 2 * l + 1 < n2;
+        float2* ca = S + P1 * (2 * l);
         float2 v[N1], u[L::E];
         any_load_pair<N>(v, ca, two ? ca + P1 : any_zero(so, P1, n2), nk1, p);
         any_warp_fft<N, true>(v, p, valid, tw2, ca, 1, u);

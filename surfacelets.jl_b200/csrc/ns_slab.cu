@@ -66,7 +66,9 @@ struct L3LoadC {
 };
 
 // The plan's NG accumulators less their compensations, summed in the
-// accumulators' order.
+// accumulators' order.  The first pass of the inverse FFT stores to the
+// accumulators it reads: plain loads there, the read-only path for the
+// compensations only.
 template <int NG>
 struct GroupSum {
     const float2* acc;
@@ -76,7 +78,7 @@ struct GroupSum {
         float2 s[NG], e[NG];
 #pragma unroll
         for (int g = 0; g < NG; ++g) {
-            s[g] = __ldg(acc + g * gstride + o);
+            s[g] = acc[g * gstride + o];
             e[g] = __ldg(comp + g * gstride + o);
         }
         float2 v = c_sub(s[0], e[0]);
