@@ -56,6 +56,13 @@ __device__ __forceinline__ void kahan_add(float2& s, float2& c, float2 v) {
     c = c_sub(c_sub(t, s), y);
     s = t;
 }
+// The same with v = a m, the product not rounded by itself.
+__device__ __forceinline__ void kahan_fma(float2& s, float2& c, float2 a, float m) {
+    const float2 y = c_fma(a, m, make_float2(-c.x, -c.y));
+    const float2 t = c_add(s, y);
+    c = c_sub(c_sub(t, s), y);
+    s = t;
+}
 // multiply by -i (forward) or +i (inverse)
 __device__ __forceinline__ float2 c_rot(float2 a, bool inv) {
     return inv ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);

@@ -8,19 +8,24 @@ namespace sfl {
 namespace {
 
 // Resident CTAs an SM the register budget aims at: three (85 registers a
-// thread) where a thread holds nine or ten values and sums, two (128) else.
-// The pass waits on L2 and gains from more warps (120 x 100 x 90 synthesis 297
-// -> 258 us), and loses far more to spilled registers (three CTAs at 128 points:
-// 489 -> 534 us).
-template <int N>
-constexpr int accum_minb() { return AnyLine<N>::N1 <= 10 && AnyLine<N>::E > 8 && AnyLine<N>::E <= 10 ? 3 : 2; }
-// Lengths whose sums go to shared memory (their register form spills).
-template <int N>
-constexpr bool accum_sums_shared() { return AnyLine<N>::E > 8; }
-template <int N>
+// thread) where a thread holds at most ten values and its sums lie in shared
+// memory, two (128) else.  The pass waits on L2 and gains from more warps (120 x
+// 100 x 90 synthesis 300 -> 257 us), and loses far more to spilled registers
+// (three CTAs at 128 points: 489 -> 534 us).
+template <int N, bool STEPS>
+constexpr int accum_minb() {
+    return AnyLine<N>::N1 <= 10 && AnyLine<N>::E > (STEPS ? 6 : 8) && AnyLine<N>::E <= 10 ? 3 : 2;
+}
+// Lengths whose sums go to shared memory: where their register form spills, and
+// with compensations from seven values on (at 64 points, sums and compensations
+// in registers at two CTAs an SM: 224 x 224 x 64 synthesis 630 us; in shared
+// memory at three: 546 us).
+template <int N, bool STEPS>
+constexpr bool accum_sums_shared() { return AnyLine<N>::E > (STEPS ? 6 : 8); }
+template <int N, bool STEPS>
 constexpr size_t accum_smem() {
-    return AnyGeom<N>::SMEM +
-           (accum_sums_shared<N>() ? (sizeof(float2) + sizeof(float)) * AnyLine<N>::E * AnyGeom<N>::THREADS : 0);
+    constexpr size_t value = STEPS ? 2 * sizeof(float2) : sizeof(float2) + sizeof(float);
+    return AnyGeom<N>::SMEM + (accum_sums_shared<N, STEPS>() ? value * AnyLine<N>::E * AnyGeom<N>::THREADS : 0);
 }
 
 // Synthesis line pass over a chunk's segments: per segment FFT_3 of every item
@@ -29,7 +34,10 @@ constexpr size_t accum_smem() {
 // compensation carries across segments and launches, so the sum over the mask
 // groups of the whole synthesis is compensated
 // (src/transforms/ns_surfacelet.jl:292, 355, 383 accumulate every subband into
-// one spectrum).  CTAs take line blocks of the union box (un) and skip the
+// one spectrum).  STEPS, the mixed pipeline: the terms of a segment are added
+// with compensation too, one Kahan step each, and the group factor multiplies
+// their sum (holding it beside the sums and compensations would leave one CTA an
+// SM at 120 points).  The compile-time slabs' sizes add them plainly.  CTAs take line blocks of the union box (un) and skip the
 // segments whose box none of their lines meets.  With several accumulators
 // (P.ngrp, blockIdx.z) mask group g goes to accumulator g mod ngrp.
 //
@@ -38,8 +46,8 @@ constexpr size_t accum_smem() {
 // sum_p wa_p(k1, k2) Y_pq, and transformed once: with nbq > 0 the segment is
 // nbq plane-b wedges q times whole rows p (item t = p nbq + q); otherwise
 // every item is its own term.  Terms are added in q order.
-template <int N>
-__global__ void __launch_bounds__(256, accum_minb<N>())
+template <int N, bool STEPS>
+__global__ void __launch_bounds__(256, accum_minb<N, STEPS>())
     ns_slab_accum_kernel(const float2* __restrict__ Y, long long ystride, int P1, int s3, BoxMap un,
                          const __grid_constant__ NSMaskTables tb, const __grid_constant__ Chunk ck, int synth,
                          float2* acc, float2* comp, const float2* __restrict__ tw, long long ychs, long long achs,
@@ -63,7 +71,7 @@ __global__ void __launch_bounds__(256, accum_minb<N>())
     float2* xl = xch + lp * Ge::XLINE;
     // a segment's sums: in registers, or (lengths whose registers would spill) in shared memory after the
     // exchange rows, value q of thread t at [q * THREADS + t]
-    constexpr bool kSumsShared = accum_sums_shared<N>();
+    constexpr bool kSumsShared = accum_sums_shared<N, STEPS>();
     float2 sr[kSumsShared ? 1 : E];
     float2* ss = xch + LP * Ge::XLINE + tid;
     auto sum = [&](int q) -> float2& {
@@ -72,8 +80,16 @@ __global__ void __launch_bounds__(256, accum_minb<N>())
         else
             return sr[q];
     };
+    // their compensations (STEPS), behind them
+    float2 cr[kSumsShared || !STEPS ? 1 : E];
+    auto rest = [&](int q) -> float2& {
+        if constexpr (kSumsShared)
+            return ss[(E + q) * Ge::THREADS];
+        else
+            return cr[q];
+    };
     // the line's group factors, in registers or beside the sums
-    float gr[kSumsShared ? 1 : E];
+    float gr[kSumsShared || STEPS ? 1 : E];
     float* gs = reinterpret_cast<float*>(xch + LP * Ge::XLINE + (kSumsShared ? E * Ge::THREADS : 0)) + tid;
     auto gf = [&](int q) -> float& {
         if constexpr (kSumsShared)
@@ -92,9 +108,12 @@ __global__ void __launch_bounds__(256, accum_minb<N>())
         // (the barrier also keeps the previous segment's exchange reads ahead of this one's writes)
         if (ck.nseg > 1 && !__syncthreads_or(valid)) continue;
 #pragma unroll
-        for (int q = 0; q < E; ++q) sum(q) = make_float2(0.f, 0.f);
+        for (int q = 0; q < E; ++q) {
+            sum(q) = make_float2(0.f, 0.f);
+            if constexpr (STEPS) rest(q) = make_float2(0.f, 0.f);
+        }
         // the group factor of the line (group table, bandpass table or the lowpass factors), once for all items
-        {
+        if constexpr (!STEPS) {
             const NSMaskLine m0 = chunk_mask_line(tb, sg, ck.item[sg.i0], k1, k2, synth != 0);
 #pragma unroll
             for (int j = 0; j < Ge::M; ++j)
@@ -156,16 +175,50 @@ __global__ void __launch_bounds__(256, accum_minb<N>())
 #pragma unroll
                 for (int k = 0; k < N2; ++k) {
                     const int k3 = Ge::has(p, j) ? (p + N2 * j) + N1 * k : 0;
-                    const float g = gf(j * N2 + k);
-                    const float m = !wedges ? g : (before ? g * mk.wb[k3 * wbs] : g * (mk.wa[k3 * was] * mk.wb[k3 * wbs]));
                     float2& tsum = sum(j * N2 + k);
-                    tsum = make_float2(fmaf(u[j * N2 + k].x, m, tsum.x), fmaf(u[j * N2 + k].y, m, tsum.y));
+                    if constexpr (STEPS) {
+                        const float m = !wedges ? 1.f : (before ? mk.wb[k3 * wbs] : mk.wa[k3 * was] * mk.wb[k3 * wbs]);
+                        kahan_fma(tsum, rest(j * N2 + k), u[j * N2 + k], m);
+                    } else {
+                        const float g = gf(j * N2 + k);
+                        const float m = !wedges ? g : (before ? g * mk.wb[k3 * wbs] : g * (mk.wa[k3 * was] * mk.wb[k3 * wbs]));
+                        tsum = make_float2(fmaf(u[j * N2 + k].x, m, tsum.x), fmaf(u[j * N2 + k].y, m, tsum.y));
+                    }
                 }
         }
         if (valid) {
             float2* a = acc + k1 + P1 * k2;
             float2* ca = comp + k1 + P1 * k2;
-            // four bins at a time: all of them at once spill
+            // a few bins at a time: all of them at once spill
+            if constexpr (STEPS) {
+                // the loads of a few bins ahead of their stores, which the compiler takes to alias
+                constexpr int B = accum_minb<N, STEPS>() == 3 ? 2 : 4;
+#pragma unroll(kSumsShared ? 1 : E)
+                for (int q0 = 0; q0 < E; q0 += B) {
+                    float2 sv[B], cv[B];
+                    float g[B];
+#pragma unroll
+                    for (int b = 0; b < B; ++b) {
+                        const int j = (q0 + b) / N2, k3 = (p + N2 * j) + N1 * (q0 + b - j * N2);
+                        if (q0 + b < E && Ge::has(p, j)) {
+                            sv[b] = a[k3 * s3];
+                            cv[b] = ca[k3 * s3];
+                            g[b] = chunk_group_factor(tb, sg, k1, k2, k3, synth != 0);
+                        }
+                    }
+#pragma unroll
+                    for (int b = 0; b < B; ++b) {
+                        const int j = (q0 + b) / N2, k3 = (p + N2 * j) + N1 * (q0 + b - j * N2);
+                        if (q0 + b < E && Ge::has(p, j)) {
+                            cv[b] = c_fma(rest(q0 + b), g[b], cv[b]);
+                            kahan_fma(sv[b], cv[b], sum(q0 + b), g[b]);
+                            a[k3 * s3] = sv[b];
+                            ca[k3 * s3] = cv[b];
+                        }
+                    }
+                }
+                continue;
+            }
 #pragma unroll(kSumsShared ? 1 : Ge::M)
             for (int j = 0; j < Ge::M; ++j)
                 if (Ge::has(p, j)) {
@@ -182,19 +235,19 @@ __global__ void __launch_bounds__(256, accum_minb<N>())
     }
 }
 
-template <int N>
+template <int N, bool STEPS>
 void launch_n(const NSPlan& P, const Chunk& ck, const BoxMap& un, int synth, const float2* Y, float2* acc, float2* comp,
               int nch, int ngrp, long long ychs, cudaStream_t st) {
     using Ge = AnyGeom<N>;
     static bool configured = false;
     if (!configured) {
-        cuda_check(cudaFuncSetAttribute(ns_slab_accum_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)accum_smem<N>()),
+        cuda_check(cudaFuncSetAttribute(ns_slab_accum_kernel<N, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)accum_smem<N, STEPS>()),
                    "cudaFuncSetAttribute");
         configured = true;
     }
     const dim3 grid((un.nk1 * un.nk2 + Ge::LP - 1) / Ge::LP, nch, ngrp);
-    ns_slab_accum_kernel<N><<<grid, Ge::THREADS, accum_smem<N>(), st>>>(
+    ns_slab_accum_kernel<N, STEPS><<<grid, Ge::THREADS, accum_smem<N, STEPS>(), st>>>(
         Y, P.SP, P.P1, P.P1 * P.dims[1], un, P.tb, ck, synth, acc, comp, P.ffts.at(N)->sh.tw, ychs, P.SP,
         (long long)P.nch * P.SP);
     cuda_check(cudaGetLastError(), "ns_slab_accum_kernel launch");
@@ -204,11 +257,21 @@ void launch_n(const NSPlan& P, const Chunk& ck, const BoxMap& un, int synth, con
 
 void launch_axis3_accum(const NSPlan& P, const Chunk& ck, const BoxMap& un, int synth, const float2* Y, float2* acc,
                         float2* comp, int nch, int ngrp, long long ychs, cudaStream_t st) {
-    switch (P.dims[2]) {
+    if (P.mixed) {
+        switch (P.dims[2]) {
 #define SFL_AXIS3_CASE(N_) \
-    case N_: launch_n<N_>(P, ck, un, synth, Y, acc, comp, nch, ngrp, ychs, st); return;
-        SFL_ANY_LENGTHS(SFL_AXIS3_CASE)
+    case N_: launch_n<N_, true>(P, ck, un, synth, Y, acc, comp, nch, ngrp, ychs, st); return;
+            SFL_ANY_LENGTHS(SFL_AXIS3_CASE)
 #undef SFL_AXIS3_CASE
+        }
+    } else {
+        switch (P.dims[2]) {   // the axis-3 lengths of the compile-time slabs (reg_fft_supported)
+#define SFL_AXIS3_CASE(N_) \
+    case N_: launch_n<N_, false>(P, ck, un, synth, Y, acc, comp, nch, ngrp, ychs, st); return;
+            SFL_AXIS3_CASE(16) SFL_AXIS3_CASE(32) SFL_AXIS3_CASE(64) SFL_AXIS3_CASE(96) SFL_AXIS3_CASE(128)
+            SFL_AXIS3_CASE(160) SFL_AXIS3_CASE(256)
+#undef SFL_AXIS3_CASE
+        }
     }
     throw ArgError("no axis-3 pass of this length");
 }

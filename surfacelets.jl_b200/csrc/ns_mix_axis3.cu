@@ -1,7 +1,7 @@
 // The axis-3 passes of the slab pipeline for any length, on the mixed-radix
 // line FFT of mixpass.cuh: the arithmetic and the tiles of the compile-time
-// passes in ns_slab.cu, with the line's X (analysis) and the segment's sums
-// (synthesis) in shared memory.
+// passes (ns_axis3_mask.cu, ns_axis3_accum.cu), with the line's X (analysis) and
+// the segment's sums (synthesis) in shared memory.
 #include <algorithm>
 
 #include "mixpass.cuh"
@@ -174,11 +174,12 @@ struct Axis3LoadTerm {
     }
 };
 
-// A transformed term times its wedge planes, added to the segment's sums.
+// A transformed term times its wedge planes, added to the segment's sums with
+// one Kahan step (their compensations lie `rest` behind them).
 struct Axis3StoreSum {
     static constexpr bool kStaged = false;
     float2* sums;
-    int pitch, l0;
+    int rest, pitch, l0;
     AxisLines ln;
     NSMaskTables tb;
     const ChunkSeg* sg;
@@ -197,17 +198,21 @@ struct Axis3StoreSum {
         return Ctx{sums + (l - l0) * pitch, m.wa, m.low || m.plain ? nullptr : m.wb, m.was, m.wbs};
     }
     __device__ __forceinline__ void put(const Ctx& c, int k, float2 v) const {
-        if (c.wb) {
-            const float w = before ? __ldg(c.wb + k * c.wbs) : __ldg(c.wa + k * c.was) * __ldg(c.wb + k * c.wbs);
-            c.s[k] = first ? c_scale(v, w) : c_fma(v, w, c.s[k]);
-        } else {
-            c.s[k] = first ? v : c_add(v, c.s[k]);
+        float w = 1.f;
+        if (c.wb) w = before ? __ldg(c.wb + k * c.wbs) : __ldg(c.wa + k * c.was) * __ldg(c.wb + k * c.wbs);
+        float2 s = make_float2(0.f, 0.f), e = s;
+        if (!first) {
+            s = c.s[k];
+            e = c.s[k + rest];
         }
+        kahan_fma(s, e, v, w);
+        c.s[k] = s;
+        c.s[k + rest] = e;
     }
 };
 
 // Synthesis axis-3 pass; segments, terms and Kahan steps as in
-// ns_slab_accum_kernel, the group factor applied to a segment's sum.
+// ns_slab_accum_kernel (STEPS), the group factor applied to a segment's sum.
 template <bool BIG>
 __global__ void __launch_bounds__(256, 2)
     ns_mix_accum_kernel(const float2* __restrict__ Y, long long ystride, const __grid_constant__ MixAxis3 g, BoxMap un,
@@ -220,8 +225,8 @@ __global__ void __launch_bounds__(256, 2)
     const int n = g.a.sc.n, LP = 1 << g.lg, tsz = g.a.pitch << g.lg;
     const int l0 = (int)blockIdx.x << g.lg, nlines = un.nk1 * un.nk2;
     const AxisLines ln{un};
-    float2* sums = sm;
-    float2* tile = sm + tsz;
+    float2* sums = sm;   // and their compensations
+    float2* tile = sm + 2 * tsz;
     const bool wedge_masks = !(synth && !tb.tight);
     // this thread's line in the Kahan steps, and its bins
     const int tt = threadIdx.x & (LP - 1);
@@ -242,7 +247,7 @@ __global__ void __launch_bounds__(256, 2)
                 mix_pass<false, BIG>(Axis3LoadTerm{Y + (it - ck.item) * ystride, ystride, g.P1, g.s3, ln, tb, it,
                                                    min(nt - p, kShare), nbq > 0 ? nbq : 1, before, sg.nk1, sg.b2,
                                                    (short)tb.n2},
-                                     Axis3StoreSum{sums, g.a.pitch, l0, ln, tb, &sg, it, synth != 0, before,
+                                     Axis3StoreSum{sums, tsz, g.a.pitch, l0, ln, tb, &sg, it, synth != 0, before,
                                                    t == 0 && p == 0},
                                      g.a, MixTile{l0, nlines, g.lg, 1}, tile, tile + tsz, tile + 2 * tsz, 0);
                 __syncthreads();
@@ -250,8 +255,9 @@ __global__ void __launch_bounds__(256, 2)
         if (in)
             for (int i = threadIdx.x >> g.lg; i < n; i += blockDim.x >> g.lg) {
                 const long long o = k1 + g.P1 * k2 + (long long)i * g.s3;
-                float2 sv = acc[o], cv = comp[o];
-                kahan_add(sv, cv, c_scale(sums[tt * g.a.pitch + i], chunk_group_factor(tb, sg, k1, k2, i, synth != 0)));
+                const float f = chunk_group_factor(tb, sg, k1, k2, i, synth != 0);
+                float2 sv = acc[o], cv = c_fma(sums[tsz + tt * g.a.pitch + i], f, comp[o]);
+                kahan_fma(sv, cv, sums[tt * g.a.pitch + i], f);
                 acc[o] = sv;
                 comp[o] = cv;
             }
@@ -259,13 +265,15 @@ __global__ void __launch_bounds__(256, 2)
     }
 }
 
-MixAxis3 mix_axis3(const NSPlan& P, size_t& smem) {
+// `beside`: tiles kept beside the FFT's own (analysis: the line's X; synthesis:
+// the sums and their compensations).
+MixAxis3 mix_axis3(const NSPlan& P, int beside, size_t& smem) {
     MixAxis3 g;
     g.a = mix_args(*P.ffts.at(P.dims[2]));
     g.P1 = P.P1;
     g.s3 = P.P1 * P.dims[1];
-    g.lg = mix_lines_lg(g.a, false, sizeof(float2) * g.a.pitch);
-    smem = mix_smem_bytes(g.a.sc, g.lg, g.a.pitch, false) + sizeof(float2) * ((size_t)g.a.pitch << g.lg);
+    g.lg = mix_lines_lg(g.a, false, beside * sizeof(float2) * g.a.pitch);
+    smem = mix_smem_bytes(g.a.sc, g.lg, g.a.pitch, false) + beside * sizeof(float2) * ((size_t)g.a.pitch << g.lg);
     return g;
 }
 
@@ -286,20 +294,20 @@ int axis3_threads(const MixAxis3& g) {
 
 bool ns_mix_slab_supported(const NSPlan& P) {
     size_t smem;
-    mix_axis3(P, smem);
+    mix_axis3(P, 2, smem);
     // 32-bit offsets within a spectrum
     return (any_slab_fits(P) || mix_slab_fits(P)) && smem <= kSlabSmemOneCta && P.SP < (1LL << 31) && P.dims[2] <= 4096;
 }
 
 int mix_axis3_lines(const NSPlan& P) {
     size_t smem;
-    return 1 << mix_axis3(P, smem).lg;
+    return 1 << mix_axis3(P, 1, smem).lg;
 }
 
 void launch_mix_mask(const NSPlan& P, const float2* X, const Chunk& ck, const MaskTiles& tl, int synth, float2* Y,
                      int nch, long long xchs, long long ychs, cudaStream_t st) {
     size_t smem;
-    const MixAxis3 g = mix_axis3(P, smem);
+    const MixAxis3 g = mix_axis3(P, 1, smem);
     const bool big = mix_big(g.a.sc);
     auto kern = big ? ns_mix_mask_kernel<true> : ns_mix_mask_kernel<false>;
     static bool configured[2] = {false, false};
@@ -311,7 +319,7 @@ void launch_mix_mask(const NSPlan& P, const float2* X, const Chunk& ck, const Ma
 void launch_mix_accum(const NSPlan& P, const Chunk& ck, const BoxMap& un, int synth, const float2* Y, float2* acc,
                       float2* comp, int nch, int ngrp, long long ychs, cudaStream_t st) {
     size_t smem;
-    const MixAxis3 g = mix_axis3(P, smem);
+    const MixAxis3 g = mix_axis3(P, 2, smem);
     const bool big = mix_big(g.a.sc);
     auto kern = big ? ns_mix_accum_kernel<true> : ns_mix_accum_kernel<false>;
     static bool configured[2] = {false, false};
