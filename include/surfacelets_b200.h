@@ -184,10 +184,12 @@ int sfl_plan_status(sfl_plan* plan, int32_t* status, int32_t reset);
  * in the reference. */
 int sfl_plan_selftest_wait(sfl_plan* plan, void* stream);
 
-/* Subbands a launch keeps in flight (NS: scratch holds that many spectra).
- * Default 8, of one mask group; left at the default, the slab pipelines put
+/* Subbands a launch keeps in flight (NS: scratch holds that many spectra, and
+ * from the first bfloat16 call that many float32 volumes).
+ * Default 8, of one mask group; while no group is set, the slab pipelines put
  * several mask groups in a launch and hold as many spectra as those take, up
- * to 256 MB.  Only affects speed and scratch size. */
+ * to 256 MB.  A group set here, 8 included, is the bound.  Only affects speed
+ * and scratch size. */
 int sfl_plan_set_group(sfl_plan* plan, int32_t group);
 
 /* NSSurfacelet kernel pipeline.  All give the same subbands to float32
@@ -221,8 +223,8 @@ int sfl_plan_tuning(const sfl_plan* plan, int32_t* pipeline, int32_t* group);
 int sfl_plan_tile(sfl_plan* plan, int32_t set, int32_t* ipc);
 
 /* Times analysis of x (into c, overwritten) followed by synthesis (into a
- * scratch volume of its own) under every pipeline that fits the size and
- * groups of 2, 4 and 8 subbands, then, on the slab pipeline, the axis-3 tile
+ * scratch volume of its own) under every pipeline that fits the size, with
+ * groups of 2 and 4 subbands and with none set, then, on the slab pipeline, the axis-3 tile
  * of 1, 2 or 4 subbands a CTA against the default 8 (sfl_plan_tile); keeps the
  * fastest and records it for the process: NS and NDFB plans created later
  * with the same transform, size and element type start with it.

@@ -146,7 +146,9 @@ void check_timeout(const sfl_plan* plan) {
     }
 }
 
-// Pipeline, group and axis-3 tile of an NS plan (the knobs of the tuner).
+// Pipeline, group (0: as it is, kDefaultGroup: none chosen) and axis-3 tile of
+// an NS plan (the knobs of the tuner).
+constexpr int kDefaultGroup = -1;
 void ns_apply(sfl::NSPlan& N, int pipeline, int group, int ipc = -1) {
     if (ipc >= 0) N.ipc = ipc;
     cudaDeviceSynchronize();
@@ -165,8 +167,12 @@ void ns_apply(sfl::NSPlan& N, int pipeline, int group, int ipc = -1) {
     } else {
         throw sfl::ArgError("unknown pipeline " + std::to_string(pipeline));
     }
-    if (group >= 1 && std::min(group, N.S) != N.group) {
-        N.group = std::min(group, N.S);
+    if (group == 0) return;
+    const bool chosen = group != kDefaultGroup;
+    const int g = std::min(chosen ? group : 8, N.S);
+    if (g != N.group || chosen != N.chosen) {
+        N.group = g;
+        N.chosen = chosen;
         sfl::ns_alloc_scratch(N);
     }
 }
@@ -545,6 +551,7 @@ int sfl_plan_set_group(sfl_plan* plan, int32_t group) {
             on_device(plan, [&] {
                 cudaDeviceSynchronize();
                 N.group = g;
+                N.chosen = true;
                 sfl::ns_alloc_scratch(N);
             });
         }
@@ -610,7 +617,7 @@ int sfl_plan_autotune(sfl_plan* plan, const void* x, void* c, void* stream) {
                 sfl::cuda_check(cudaEventElapsedTime(&ms, e0, e1), "cudaEventElapsedTime");
                 return ms;
             };
-            Tuning pick{ns_pipeline_of(N), N.group, N.ipc};
+            Tuning pick{ns_pipeline_of(N), N.chosen ? N.group : kDefaultGroup, N.ipc};
             float best = 1e30f;
             try {
                 std::vector<int> pipes;
@@ -620,7 +627,7 @@ int sfl_plan_autotune(sfl_plan* plan, const void* x, void* c, void* stream) {
                 // pipeline x group at the default tile, then the slab tile (subbands a CTA of the axis-3
                 // analysis pass) for the best group
                 for (int pipe : pipes)
-                    for (int g : {2, 4, 8}) {
+                    for (int g : {2, 4, kDefaultGroup}) {
                         if (g > N.S && g != 2) continue;
                         const float ms = time_it(pipe, g, 0);
                         if (ms < best) {

@@ -552,11 +552,11 @@ NSBox ns_table_box(const std::vector<double>& g, int h1, int n2, int n3) {
 
 // Work slots of the slab pipeline: the group when one was chosen, else as many
 // spectra as 256 MB hold (complex volumes: two channels each), so that a chunk
-// spans the mask groups of small boxes.
-// No more than the transforms' own chunks use.
+// spans the mask groups of small boxes; no more than the transforms' own
+// chunks use.
 void ns_slab_slots(NSPlan& P) {
     P.slots = P.group;
-    if (P.group != std::min(8, P.S)) return;
+    if (P.chosen) return;
     const long long fit = (256LL << 20) / (8 * P.SP * P.nch);
     P.slots = (int)std::max<long long>(P.group, std::min<long long>({fit, (long long)kChunkItems, (long long)P.S}));
     int used = P.group;

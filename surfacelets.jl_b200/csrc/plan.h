@@ -128,6 +128,7 @@ struct NSPlan {
     int S = 0;            // subbands
     int nch = 1;          // 1 real, 2 complex
     bool ndfb = false;    // the standalone directional bank (no pyramid, no lowpass)
+    bool chosen = false;  // the group was chosen (by the caller or the tuner): it bounds the work spectra
     int group = 8;
     int slots = 8;        // work spectra: subbands in flight per launch (the slab pipeline's chunks)
     int ipc = 0;          // subbands a CTA of the slab axis-3 analysis pass takes (1, 2, 4, 8; 0: the default, mask_ipc)
