@@ -199,8 +199,10 @@ int sfl_plan_set_group(sfl_plan* plan, int32_t group);
  *     along axis 3 plus one pass per axis-3 slab, skipping the zero rows and
  *     columns of band-limited masks.
  *   MIXED (default for the other lengths whose slabs fit shared memory, about
- *     216 x 216 and, with more room, odd and prime lengths too): the same two
- *     passes on a mixed-radix FFT.
+ *     216 x 216 and, with more room, odd and prime lengths too; not where one
+ *     axis is above 256, or axis 3 above 512, and the others are 16, 32, 64,
+ *     96, 128, 160 or 256, which lines run faster): the same two passes on a
+ *     mixed-radix FFT.
  *   LINES (default elsewhere): one line pass per axis.
  *   PLANES: retired (the plane-major pipeline was slower than SLABS at every
  *     size it supported); selecting it returns SFL_ERR_ARGUMENT.

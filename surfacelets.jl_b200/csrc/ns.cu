@@ -279,6 +279,24 @@ static std::vector<float> to_f32(const std::vector<double>& v) {
     return o;
 }
 
+// Whether the line pipeline is the faster one although the slabs would fit: one
+// axis too long for the slab passes' compile-time lengths (run-time radices,
+// one slab an SM: above 256; axis 3 above 512) while every other axis has a
+// compile-time line pass.  Synthesis at 512 x 64 x 32: 257 us on lines, 411
+// mixed; 32 x 400 x 32: 141 and 220; analysis at 16 x 16 x 1000: 144 and 170.
+// With other lengths beside it the mixed pipeline is ahead (280 x 140 x 28
+// analysis: 455 and 263; 20 x 20 x 700: 195 and 156).
+static bool ns_lines_ahead(const int dims[3]) {
+    bool longer = false;
+    for (int d = 0; d < 3; ++d) {
+        if (dims[d] > (d == 2 ? 512 : 256))
+            longer = true;
+        else if (!reg_fft_supported(dims[d]))
+            return false;
+    }
+    return longer;
+}
+
 // With ndfb, the standalone directional bank of one level count
 // (src/directional/ndfb.jl:91-104; HourglassFB at level 0): the same cascade
 // with the hourglass masks alone as group factors, no pyramid and no lowpass.
@@ -402,7 +420,7 @@ void ns_plan_init(NSPlan& P, const sfl_ns_params& p, const int dims[3], int dtyp
     while (P.P1 % 4 != 2) ++P.P1;
     P.SP = (long long)P.P1 * dims[1] * dims[2];
     P.slab = ns_slab_supported(dims[0], dims[1], dims[2]);
-    if (!P.slab) P.slab = P.mixed = ns_mix_slab_supported(P);
+    if (!P.slab && !ns_lines_ahead(dims)) P.slab = P.mixed = ns_mix_slab_supported(P);
     ns_alloc_scratch(P);
 }
 

@@ -1,0 +1,31 @@
+"""The pipeline a plan starts with, and the ones that can be selected: a long
+axis beside lengths with compile-time line passes takes lines (where the mixed
+pipeline is slower), other lengths the mixed pipeline where the slabs fit;
+either gives the same subbands."""
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dims,default", [
+    ((256, 20, 32), "mixed"), ((258, 32, 32), "lines"), ((258, 20, 32), "mixed"), ((32, 257, 16), "lines"),
+    ((16, 32, 512), "mixed"), ((16, 32, 513), "lines"), ((16, 18, 513), "mixed"), ((512, 64, 32), "lines"),
+    ((32, 400, 32), "lines"), ((16, 16, 1000), "lines"), ((64, 64, 64), "slabs"), ((250, 250, 20), "lines"),
+])
+def test_default_pipeline(sfl, dims, default):
+    t = sfl.NSSurfacelet(direction_levels=[1], bernstein_order=4)
+    ws = sfl.make_workspace(t, "float32", dims)
+    assert ws.tuning()[0] == default
+    if default == "slabs" or dims[:2] == (250, 250):
+        return
+    other = sfl.make_workspace(t, "float32", dims)
+    other.set_pipeline("lines" if default == "mixed" else "mixed")   # both stay selectable
+    x = sfl.to_device(np.random.default_rng(3).standard_normal(dims).astype(np.float32))
+    a, b = sfl.analyze(ws, x), sfl.analyze(other, x)
+    # two orders of the same float32 transform: each within about 3e-7 of 64 bits
+    assert float(torch.linalg.vector_norm(a - b) / torch.linalg.vector_norm(a)) <= 1e-6
+    y, z = sfl.synthesize(ws, a), sfl.synthesize(other, a)
+    assert float(torch.linalg.vector_norm(y - z) / torch.linalg.vector_norm(y)) <= 1e-6
