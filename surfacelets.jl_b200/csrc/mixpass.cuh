@@ -457,7 +457,11 @@ template <bool INV, bool BIG, class Load, class Store>
 void launch_mix_b(const FFTLen& f, const Load& ld, const Store& st, int nlines, int nz, bool tfast,
                   cudaStream_t stream, const char* tag) {
     const MixArgs a = mix_args(f);
-    const int lg = mix_lines_lg(a, Store::kStaged);
+    int lg = mix_lines_lg(a, Store::kStaged);
+    // Tiles of long lines are large, and a small volume has few: fewer lines a tile (strided ones keep 32-byte
+    // runs) until every SM has two CTAs.  C2R of 1000 x 16 x 16, 8 subbands: 26 us a launch in 128 tiles of 8 lines.
+    if (a.sc.n > 256)
+        while (lg > (tfast ? 2 : 0) && (long long)((nlines + (1 << lg) - 1) >> lg) * nz < 2 * 148) --lg;
     const size_t smem = mix_smem_bytes(a.sc, lg, a.pitch, Store::kStaged);
     auto kern = mix_pass_kernel<INV, BIG, Load, Store>;
     static bool configured = false;

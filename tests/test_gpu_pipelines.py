@@ -7,6 +7,8 @@ import numpy as np
 import pytest
 import torch
 
+from oracle import ns as N
+
 pytestmark = pytest.mark.gpu
 
 
@@ -29,3 +31,20 @@ def test_default_pipeline(sfl, dims, default):
     assert float(torch.linalg.vector_norm(a - b) / torch.linalg.vector_norm(a)) <= 1e-6
     y, z = sfl.synthesize(ws, a), sfl.synthesize(other, a)
     assert float(torch.linalg.vector_norm(y - z) / torch.linalg.vector_norm(y)) <= 1e-6
+
+
+@pytest.mark.parametrize("dims", [(1000, 8, 8), (10, 600, 12), (12, 6, 520), (521, 8, 10), (8, 8, 541), (258, 34, 6)])
+def test_long_lines_in_small_tiles(sfl, dims):
+    """Few long lines run in tiles of one to eight lines: against the float64
+    oracle, bar 1e-5 (float32 rounding measures 2e-7 to 5e-7)."""
+    kw = dict(direction_levels=[1], bernstein_order=4)
+    rng = np.random.default_rng(8)
+    x = rng.standard_normal(dims).astype(np.float32)
+    T = N.make_tables(N.NSParams.make(**kw), dims)
+    ws = sfl.make_workspace(sfl.NSSurfacelet(**kw), "float32", dims)
+    ws.set_pipeline("lines")
+    ref = N.analyze(T, x)
+    c = rng.standard_normal(ref.shape).astype(np.float32)
+    assert np.linalg.norm(sfl.to_host(sfl.analyze(ws, sfl.to_device(x))) - ref) <= 1e-5 * np.linalg.norm(ref)
+    y = N.synthesize(T, c)
+    assert np.linalg.norm(sfl.to_host(sfl.synthesize(ws, sfl.to_device(c))) - y) <= 1e-5 * np.linalg.norm(y)
