@@ -21,6 +21,9 @@
 // and q - m together (half the products of the direct sum).
 #pragma once
 
+#include <type_traits>
+#include <utility>
+
 #include "passes.cuh"
 #include "plan.h"
 #include "prof.h"
@@ -412,9 +415,12 @@ inline size_t mix_smem_bytes(const MixSchedule& sc, int lg, int pitch, bool stag
     return sizeof(float2) * (((size_t)pitch << lg) * (big || staged ? 2 : 1) + (big ? sc.R[0] : 0));
 }
 
-inline MixArgs mix_args(const FFTLen& f) {
+// small_first: the smaller of two radices first, so that the first step's loads
+// spread over more threads.
+inline MixArgs mix_args(const FFTLen& f, bool small_first = false) {
     MixArgs a;
-    const MixSchedule& sc = f.mix;
+    MixSchedule sc = f.mix;
+    if (small_first && sc.ns == 2 && sc.R[0] <= 16 && sc.R[0] > sc.R[1]) std::swap(sc.R[0], sc.R[1]);
     a.sc = sc;
     a.tw = f.sh.tw;
     a.rev = sc.ns > 2 ? f.rev.as<unsigned short>() : nullptr;
@@ -453,11 +459,23 @@ inline int mix_threads(const MixArgs& a, int lg) {
     return std::min(256, std::max(t, least));
 }
 
+// Load ops with several reads and products a value (Load::kHeavy: the masked
+// axis-3 load).  The first step is where they run, so it takes the smaller radix
+// of two (256 x 256 x 75 analysis, 5 x 15 for 15 x 5: 1825 -> 1083 us; 27
+// 622 -> 412) and tiles of one round of items (63 points: 1049 -> 827).
+template <class Load, class = void>
+struct HeavyLoad : std::false_type {};
+template <class Load>
+struct HeavyLoad<Load, std::void_t<decltype(Load::kHeavy)>> : std::bool_constant<Load::kHeavy> {};
+
 template <bool INV, bool BIG, class Load, class Store>
 void launch_mix_b(const FFTLen& f, const Load& ld, const Store& st, int nlines, int nz, bool tfast,
                   cudaStream_t stream, const char* tag) {
-    const MixArgs a = mix_args(f);
+    const MixArgs a = mix_args(f, HeavyLoad<Load>::value);
     int lg = mix_lines_lg(a, Store::kStaged);
+    // heavy loads: one round of the widest step rather than a second one for a few items
+    if (HeavyLoad<Load>::value)
+        while (lg > 4 && (mix_items(a.sc) << lg) > 256) --lg;
     // Tiles of long lines are large, and a small volume has few: fewer lines a tile (strided ones keep 32-byte
     // runs) until every SM has two CTAs.  C2R of 1000 x 16 x 16, 8 subbands: 26 us a launch in 128 tiles of 8 lines.
     if (a.sc.n > 256)

@@ -67,6 +67,7 @@ __device__ __forceinline__ float ns_mask_at(const NSMaskLine& c, int k3, long lo
 
 // Analysis pass-3 load for the register kernel: X times the mask of item z.
 struct RLoadNSMask {
+    static constexpr bool kHeavy = true;
     const float2* X;
     NSMaskTables tb;
     const NSItem* items;

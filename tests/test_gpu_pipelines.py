@@ -48,3 +48,15 @@ def test_long_lines_in_small_tiles(sfl, dims):
     assert np.linalg.norm(sfl.to_host(sfl.analyze(ws, sfl.to_device(x))) - ref) <= 1e-5 * np.linalg.norm(ref)
     y = N.synthesize(T, c)
     assert np.linalg.norm(sfl.to_host(sfl.synthesize(ws, sfl.to_device(c))) - y) <= 1e-5 * np.linalg.norm(y)
+
+
+@pytest.mark.parametrize("n3", [6, 18, 20, 27, 34, 40, 45, 60, 63, 75, 90, 108, 143, 150, 208, 225])
+def test_masked_lines_of_two_radices(sfl, n3):
+    """The line pipeline's masked axis-3 pass takes the smaller radix first:
+    against the float64 oracle (bar 1e-5), ragged counts of lines."""
+    dims, kw = (22, 18, n3), dict(direction_levels=[1], bernstein_order=4)
+    x = np.random.default_rng(9).standard_normal(dims).astype(np.float32)
+    ws = sfl.make_workspace(sfl.NSSurfacelet(**kw), "float32", dims)
+    ws.set_pipeline("lines")
+    ref = N.analyze(N.make_tables(N.NSParams.make(**kw), dims), x)
+    assert np.linalg.norm(sfl.to_host(sfl.analyze(ws, sfl.to_device(x))) - ref) <= 1e-5 * np.linalg.norm(ref)
