@@ -1064,14 +1064,9 @@ IrcPlaneStages irc_plane_stages(const DecLevelDev& L, int K, bool synth) {
 }
 
 template <bool SYNTH>
-void irc_plane_configure(size_t smem) {
-    static size_t configured = 0;
-    if (smem > configured) {
-        cuda_check(cudaFuncSetAttribute(irc_plane_kernel<SYNTH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem),
-                   "cudaFuncSetAttribute(irc_plane)");
-        configured = smem;
-    }
+void irc_plane_configure() {
+    static DeviceOnce once;
+    allow_smem(once, irc_plane_kernel<SYNTH>, 227 * 1024);
 }
 
 // Whether the plane pass of level L runs hourglass K (its plane fits; the
@@ -1097,7 +1092,7 @@ void irc_plane_launch_levels(DecPlan& D, cudaStream_t st, bool adjoint = false) 
     int blocks = 0;
     auto flush = [&] {
         if (jobs.n == 0) return;
-        irc_plane_configure<SYNTH>(smem);
+        irc_plane_configure<SYNTH>();
         int tok = prof_begin("dec_irc_plane", st);
         irc_plane_kernel<SYNTH><<<blocks, kIrcPlaneThreads, smem, st>>>(jobs);
         prof_end(tok, st);

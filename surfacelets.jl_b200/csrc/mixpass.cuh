@@ -462,7 +462,7 @@ inline int mix_threads(const MixArgs& a, int lg) {
 // Load ops with several reads and products a value (Load::kHeavy: the masked
 // axis-3 load).  The first step is where they run, so it takes the smaller radix
 // of two (256 x 256 x 75 analysis, 5 x 15 for 15 x 5: 1825 -> 1083 us; 27
-// 622 -> 412) and tiles of one round of items (63 points: 1049 -> 827).
+// points: 622 -> 505) and tiles of one round of items (505 -> 408).
 template <class Load, class = void>
 struct HeavyLoad : std::false_type {};
 template <class Load>
@@ -482,12 +482,8 @@ void launch_mix_b(const FFTLen& f, const Load& ld, const Store& st, int nlines, 
         while (lg > (tfast ? 2 : 0) && (long long)((nlines + (1 << lg) - 1) >> lg) * nz < 2 * 148) --lg;
     const size_t smem = mix_smem_bytes(a.sc, lg, a.pitch, Store::kStaged);
     auto kern = mix_pass_kernel<INV, BIG, Load, Store>;
-    static bool configured = false;
-    if (!configured) {
-        cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
-                   "cudaFuncSetAttribute(mix)");
-        configured = true;
-    }
+    static DeviceOnce once;
+    allow_smem(once, kern, 227 * 1024);
     const dim3 grid((unsigned)((nlines + (1 << lg) - 1) >> lg), (unsigned)nz);
     int tok = prof_begin(tag, stream);
     kern<<<grid, mix_threads(a, lg), smem, stream>>>(ld, st, a, nlines, lg, tfast ? 1 : 0);

@@ -157,13 +157,8 @@ static void launch_accum_reg(const float2* W, long long H, int nz, const NSMaskT
                              int i0, int synth, float2* acc, float2* comp, int init, const float2* tw, int nlines,
                              cudaStream_t st) {
     using Ge = RegGeom<N>;
-    static bool configured = false;
-    if (!configured) {
-        cuda_check(cudaFuncSetAttribute(ns_accum_reg_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)Ge::SMEM),
-                   "cudaFuncSetAttribute");
-        configured = true;
-    }
+    static DeviceOnce once;
+    allow_smem(once, ns_accum_reg_kernel<N>, Ge::SMEM);
     dim3 grid((nlines + Ge::LP - 1) / Ge::LP);
     int tok = prof_begin("ns_accum_axis3", st);
     ns_accum_reg_kernel<N><<<grid, Ge::THREADS, Ge::SMEM, st>>>(W, H, nz, tb, items, i0, synth, acc, comp, init, tw,
@@ -563,12 +558,8 @@ void accum_items(NSPlan& P, int i0, int nz, bool analysis_masks, float2* acc, fl
     const int lg = mix_lines_lg(a, false, 2 * sizeof(float2) * (n + 1)), nlines = P.h1 * P.dims[1];
     const size_t smem = mix_smem_bytes(a.sc, lg, a.pitch, false) + 2 * sizeof(float2) * ((size_t)a.pitch << lg);
     auto kern = big ? ns_accum_mix_kernel<true> : ns_accum_mix_kernel<false>;
-    static bool configured[2] = {false, false};
-    if (!configured[big]) {
-        cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
-                   "cudaFuncSetAttribute");
-        configured[big] = true;
-    }
+    static DeviceOnce once[2];
+    allow_smem(once[big], kern, 227 * 1024);
     int tok = prof_begin("ns_accum_axis3", st);
     kern<<<(nlines + (1 << lg) - 1) >> lg, mix_threads(a, lg), smem, st>>>(
         W, P.H, nz, P.tb, P.items.as<NSItem>(), i0, analysis_masks ? 0 : 1, acc, comp, init ? 1 : 0, a, nlines, lg);
@@ -637,13 +628,8 @@ template <int N>
 void launch_shrink_axis1(const RLoadHPair& ld, const RStoreHalfPair& sto, const float2* tw, int nlines, int nz,
                          float scale, const float* tau, const NSItem* items, int item0, cudaStream_t st) {
     using G = RegGeom<N>;
-    static bool configured = false;
-    if (!configured) {
-        cuda_check(cudaFuncSetAttribute(reg_shrink_axis1_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)G::SMEM),
-                   "cudaFuncSetAttribute");
-        configured = true;
-    }
+    static DeviceOnce once;
+    allow_smem(once, reg_shrink_axis1_kernel<N>, G::SMEM);
     dim3 grid((nlines + G::LP - 1) / G::LP, nz);
     int tok = prof_begin("ns_shrink_axis1", st);
     reg_shrink_axis1_kernel<N><<<grid, G::THREADS, G::SMEM, st>>>(ld, sto, tw, nlines, scale, tau, items, item0);

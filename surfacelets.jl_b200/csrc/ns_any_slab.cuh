@@ -439,12 +439,8 @@ inline int any_warps(int n1, int n2, size_t smem) {
 template <int KIND, int ES>
 void launch_any_slab_es(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char* tag) {
     auto kern = ns_any_slab_kernel<KIND, ES>;
-    static bool configured = false;
-    if (!configured) {
-        cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmemOneCta),
-                   "cudaFuncSetAttribute(any slab)");
-        configured = true;
-    }
+    static DeviceOnce once;
+    allow_smem(once, kern, kSlabSmemOneCta);
     const int n1 = P.dims[0], n2 = P.dims[1];
     const size_t smem = any_smem(n1, n2, a.P1);
     const int threads = 32 * any_warps(n1, n2, smem);

@@ -239,13 +239,8 @@ template <int N, bool STEPS>
 void launch_n(const NSPlan& P, const Chunk& ck, const BoxMap& un, int synth, const float2* Y, float2* acc, float2* comp,
               int nch, int ngrp, long long ychs, cudaStream_t st) {
     using Ge = AnyGeom<N>;
-    static bool configured = false;
-    if (!configured) {
-        cuda_check(cudaFuncSetAttribute(ns_slab_accum_kernel<N, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)accum_smem<N, STEPS>()),
-                   "cudaFuncSetAttribute");
-        configured = true;
-    }
+    static DeviceOnce once;
+    allow_smem(once, ns_slab_accum_kernel<N, STEPS>, accum_smem<N, STEPS>());
     const dim3 grid((un.nk1 * un.nk2 + Ge::LP - 1) / Ge::LP, nch, ngrp);
     ns_slab_accum_kernel<N, STEPS><<<grid, Ge::THREADS, accum_smem<N, STEPS>(), st>>>(
         Y, P.SP, P.P1, P.P1 * P.dims[1], un, P.tb, ck, synth, acc, comp, P.ffts.at(N)->sh.tw, ychs, P.SP,

@@ -111,13 +111,8 @@ template <int N>
 void launch_n(const NSPlan& P, const float2* X, const Chunk& ck, const MaskTiles& tl, int synth, float2* Y, int nch,
               long long xchs, long long ychs, cudaStream_t st) {
     using Ge = AnyGeom<N>;
-    static bool configured = false;
-    if (!configured) {
-        cuda_check(cudaFuncSetAttribute(ns_slab_mask_group_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)Ge::SMEM),
-                   "cudaFuncSetAttribute");
-        configured = true;
-    }
+    static DeviceOnce once;
+    allow_smem(once, ns_slab_mask_group_kernel<N>, Ge::SMEM);
     ns_slab_mask_group_kernel<N><<<dim3(tl.first[tl.n], nch), Ge::THREADS, Ge::SMEM, st>>>(
         X, P.P1, P.P1 * P.dims[1], P.tb, ck, tl, synth, Y, P.SP, P.ffts.at(N)->sh.tw, xchs, ychs);
     cuda_check(cudaGetLastError(), "ns_slab_mask_group_kernel launch");

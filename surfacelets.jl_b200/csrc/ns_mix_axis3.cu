@@ -277,14 +277,6 @@ MixAxis3 mix_axis3(const NSPlan& P, int beside, size_t& smem) {
     return g;
 }
 
-template <class K>
-void allow_smem(K kern, bool& configured) {
-    if (configured) return;
-    cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmemOneCta),
-               "cudaFuncSetAttribute(mix axis 3)");
-    configured = true;
-}
-
 int axis3_threads(const MixAxis3& g) {
     // a whole number of threads a line
     return std::max(1 << g.lg, mix_threads(g.a, g.lg) >> g.lg << g.lg);
@@ -310,8 +302,8 @@ void launch_mix_mask(const NSPlan& P, const float2* X, const Chunk& ck, const Ma
     const MixAxis3 g = mix_axis3(P, 1, smem);
     const bool big = mix_big(g.a.sc);
     auto kern = big ? ns_mix_mask_kernel<true> : ns_mix_mask_kernel<false>;
-    static bool configured[2] = {false, false};
-    allow_smem(kern, configured[big]);
+    static DeviceOnce once[2];
+    allow_smem(once[big], kern, kSlabSmemOneCta);
     kern<<<dim3(tl.first[tl.n], nch), axis3_threads(g), smem, st>>>(X, g, P.tb, ck, tl, synth, Y, P.SP, xchs, ychs);
     cuda_check(cudaGetLastError(), "ns_mix_mask_kernel launch");
 }
@@ -322,8 +314,8 @@ void launch_mix_accum(const NSPlan& P, const Chunk& ck, const BoxMap& un, int sy
     const MixAxis3 g = mix_axis3(P, 2, smem);
     const bool big = mix_big(g.a.sc);
     auto kern = big ? ns_mix_accum_kernel<true> : ns_mix_accum_kernel<false>;
-    static bool configured[2] = {false, false};
-    allow_smem(kern, configured[big]);
+    static DeviceOnce once[2];
+    allow_smem(once[big], kern, kSlabSmemOneCta);
     const int lines = un.nk1 * un.nk2;
     kern<<<dim3((lines + (1 << g.lg) - 1) >> g.lg, nch, ngrp), axis3_threads(g), smem, st>>>(
         Y, P.SP, g, un, P.tb, ck, synth, acc, comp, ychs, P.SP, (long long)P.nch * P.SP);

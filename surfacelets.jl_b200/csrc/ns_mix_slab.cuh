@@ -268,12 +268,8 @@ bool mix_slab_geom(const MixArgs& a1, const MixArgs& a2, int P1, int kind, MixSl
 template <int KIND, bool BIG>
 void launch_mix_slab_b(const SlabArgs& a, const MixSlabGeom& g, int sms, cudaStream_t st, const char* tag) {
     auto kern = ns_mix_slab_kernel<KIND, BIG>;
-    static bool configured = false;
-    if (!configured) {
-        cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmemOneCta),
-                   "cudaFuncSetAttribute(mix slab)");
-        configured = true;
-    }
+    static DeviceOnce once;
+    allow_smem(once, kern, kSlabSmemOneCta);
     const size_t smem = mix_slab_smem(g, a.P1, KIND);
     const int items = std::max(mix_items(g.a1.sc), mix_items(g.a2.sc)) << g.lg;
     const int threads = std::min(kMixSlabThreads, std::max(64, (items + 31) / 32 * 32));

@@ -24,6 +24,7 @@
 //            both CTAs' rows; | FFT_2 own rows, out.
 // (| = cluster barrier.)
 #include <algorithm>
+#include <atomic>
 #include <cooperative_groups.h>
 
 #include "prof.h"
@@ -390,8 +391,8 @@ void launch_cluster(const SlabArgs& a, int sms, cudaStream_t st, const char* tag
     using C = ClusterSlab<NA, NB>;
     auto kern = KIND == 1 ? ns_slab_cluster_inv_kernel<NA, NB, ES>
                           : (KIND == 0 ? ns_slab_cluster_fwd_kernel<NA, NB, ES> : ns_slab_cluster_shrink_kernel<NA, NB>);
-    static bool configured = false;
-    static int max_clusters = 0;
+    static DeviceOnce once;
+    static std::atomic<int> max_clusters{1};   // the same on every device of sm_100a
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -403,16 +404,16 @@ void launch_cluster(const SlabArgs& a, int sms, cudaStream_t st, const char* tag
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (!configured) {
+    once_a_device(once, [&] {
         cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM),
                    "cudaFuncSetAttribute(cluster slab)");
         cfg.gridDim = dim3(kClusterCTAs * (unsigned)std::max(1, sms / kClusterCTAs));
-        cuda_check(cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg),
-                   "cudaOccupancyMaxActiveClusters(cluster slab)");
-        if (max_clusters < 1) throw ArgError("the cluster slab kernel cannot be resident on this device");
-        configured = true;
-    }
-    const int nclusters = std::max(1, std::min(a.units, max_clusters));
+        int n = 0;
+        cuda_check(cudaOccupancyMaxActiveClusters(&n, kern, &cfg), "cudaOccupancyMaxActiveClusters(cluster slab)");
+        if (n < 1) throw ArgError("the cluster slab kernel cannot be resident on this device");
+        max_clusters = n;
+    });
+    const int nclusters = std::max(1, std::min(a.units, max_clusters.load()));
     cfg.gridDim = dim3((unsigned)(kClusterCTAs * nclusters));
     int tok = prof_begin(tag, st);
     cuda_check(cudaLaunchKernelEx(&cfg, kern, a), "cluster slab kernel launch");

@@ -4,6 +4,7 @@
 #pragma once
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "plan.h"
@@ -504,16 +505,16 @@ void launch_slab_es(const SlabArgs& a, int sms, size_t smem, cudaStream_t st, co
     constexpr int MINB = (slab_minb<NA>() == 2 && slab_minb<NB>() == 2) ? 2 : 1;
     auto kern = KIND == 1 ? ns_slab_inv_kernel<NA, NB, ES, MINB>
                           : (KIND == 0 ? ns_slab_fwd_kernel<NA, NB, ES, MINB> : ns_slab_shrink_kernel<NA, NB, MINB>);
-    static size_t configured = 0;
-    static int resident = 0;
-    if (configured < smem) {
+    static DeviceOnce once;
+    static std::atomic<int> resident{1};   // the same on every device of sm_100a
+    once_a_device(once, [&] {
         cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                    "cudaFuncSetAttribute(slab)");
-        configured = smem;
-        cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, kSlabThreads, smem),
+        int r = 0;
+        cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kern, kSlabThreads, smem),
                    "cudaOccupancyMaxActiveBlocksPerMultiprocessor(slab)");
-        resident = std::max(resident, 1);
-    }
+        resident = std::max(r, 1);
+    });
     const int grid = std::max(1, std::min(a.units, resident * sms));
     int tok = prof_begin(tag, st);
     kern<<<grid, kSlabThreads, smem, st>>>(a);

@@ -8,6 +8,7 @@
 #include <string>
 #include <vector>
 
+#include "device_once.h"
 #include "design.h"
 #include "fft_core.cuh"
 
@@ -28,6 +29,23 @@ struct TimeoutError : std::runtime_error {
 };
 
 void cuda_check(cudaError_t e, const char* what);
+
+// f() once for the calling thread's device.
+template <class F>
+void once_a_device(DeviceOnce& once, F&& f) {
+    int dev = 0;
+    cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+    once.run(dev, f);
+}
+
+// Allows a kernel that much dynamic shared memory.
+template <class K>
+void allow_smem(DeviceOnce& once, K kern, size_t bytes) {
+    once_a_device(once, [&] {
+        cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes),
+                   "cudaFuncSetAttribute");
+    });
+}
 
 // Device allocation owned by a plan.
 // One int in mapped, page-locked host memory: kernels store to it through

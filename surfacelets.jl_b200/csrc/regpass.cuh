@@ -312,13 +312,8 @@ template <int N, bool INV, class Load, class Store>
 void launch_reg_n(const Load& ld, const Store& st, const float2* tw, int nlines, int nz, bool tfast,
                   cudaStream_t stream, const char* tag) {
     using G = RegGeom<N>;
-    static bool configured = false;
-    if (!configured) {
-        cuda_check(cudaFuncSetAttribute(reg_pass_kernel<N, INV, Load, Store>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM),
-                   "cudaFuncSetAttribute");
-        configured = true;
-    }
+    static DeviceOnce once;
+    allow_smem(once, reg_pass_kernel<N, INV, Load, Store>, G::SMEM);
     dim3 grid((nlines + G::LP - 1) / G::LP, nz);
     int tok = prof_begin(tag, stream);
     reg_pass_kernel<N, INV, Load, Store><<<grid, G::THREADS, G::SMEM, stream>>>(ld, st, tw, nlines, tfast ? 1 : 0);
