@@ -4,7 +4,7 @@
 namespace sfl {
 
 void launch_mix_slab_inv(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char* tag) {
-    launch_mix_slab_kind<1>(P, a, st, tag);
+    launch_mix_slab_kind<kMixInv>(P, a, st, tag);
 }
 
 }  // namespace sfl

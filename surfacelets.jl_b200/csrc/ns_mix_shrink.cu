@@ -4,7 +4,8 @@
 namespace sfl {
 
 void launch_mix_slab_shrink(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char* tag) {
-    launch_mix_slab_kind<2>(P, a, st, tag);
+    launch_mix_slab_kind<kMixShrink>(P, a, st, tag);
+    launch_mix_slab_kind<kMixUnshrink>(P, a, st, tag);
 }
 
 }  // namespace sfl

@@ -117,29 +117,25 @@ struct ColStoreReal {
         if (c.b) c.b[k * es] = w.y;
     }
 };
-// The same two real lines, soft-thresholded, into a tile (the denoiser).
+// The same two real lines, soft-thresholded (the denoiser).
 struct ColStoreShrink {
     static constexpr bool kStaged = false;
-    float2* tile;
-    int pitch, l0;
+    float* out;
+    int n1, n2;
     float scale, tau;
     struct Ctx {
-        float2* p;
+        float* a;
+        float* b;
     };
-    __device__ __forceinline__ Ctx line(int, int l, bool) const { return Ctx{tile + (l - l0) * pitch}; }
+    __device__ __forceinline__ Ctx line(int, int l, bool) const {
+        float* a = out + 2 * l * n1;
+        return Ctx{a, 2 * l + 1 < n2 ? a + n1 : nullptr};
+    }
     __device__ __forceinline__ void put(const Ctx& c, int k, float2 v) const {
         const float2 x = c_scale(v, scale);
-        c.p[k] = make_float2(copysignf(fmaxf(fabsf(x.x) - tau, 0.f), x.x), copysignf(fmaxf(fabsf(x.y) - tau, 0.f), x.y));
+        c.a[k] = copysignf(fmaxf(fabsf(x.x) - tau, 0.f), x.x);
+        if (c.b) c.b[k] = copysignf(fmaxf(fabsf(x.y) - tau, 0.f), x.y);
     }
-};
-struct ColLoadTile {
-    const float2* tile;
-    int pitch, l0;
-    struct Ctx {
-        const float2* p;
-    };
-    __device__ __forceinline__ Ctx line(int, int l, bool valid) const { return Ctx{tile + (valid ? l - l0 : 0) * pitch}; }
-    __device__ __forceinline__ float2 get(const Ctx& c, int i) const { return c.p[i]; }
 };
 // Two real columns of a volume as one complex line, and its spectrum unpacked
 // into the slab's columns (rows of the box).
@@ -197,7 +193,14 @@ __device__ __forceinline__ void mix_lines(const Load& ld, const Store& st, const
     }
 }
 
-// KIND: 0 the forward slab pass, 1 the inverse, 2 the denoiser's shrink pass.
+// The slab passes of the run-time radices.  The denoiser runs two: the inverse
+// one with thresholded stores into the slab's own block of the spectrum (its
+// reals take at most half the block, and its CTA has read the block by then),
+// and the forward one from there.  As one pass with three tiles a CTA it was
+// slower than the two apart: 64 x 200 x 64 denoised 515 -> 411 us, 127 x 127 x 64
+// 1889 -> 1082.
+enum MixSlabKind { kMixFwd, kMixInv, kMixShrink, kMixUnshrink };
+
 // One CTA a unit (channel, item, n3), striding over the launch's units.
 template <int KIND, bool BIG>
 __global__ void __launch_bounds__(kMixSlabThreads, 2)
@@ -216,51 +219,49 @@ __global__ void __launch_bounds__(kMixSlabThreads, 2)
         float2* slab = a.spec + ch * a.spec_chstride + z * a.spec_zstride + s3 * SL;
         // narrow boxes take half tiles, so that fewer lanes hold no row
         const int lgr = g.lg > 4 && nk1 <= 16 ? 4 : g.lg;
-        if constexpr (KIND != 0)
-            mix_lines<true, BIG>(RowLoadBox{slab, P1, b2, k2hi}, RowStoreS{S, P1}, g.a2, nk1, lgr, 1, tile, g.tsz);
-        if constexpr (KIND == 0) {
+        constexpr bool kFwd = KIND == kMixFwd || KIND == kMixUnshrink;
+        if constexpr (kFwd) {
             const float* in = a.vol + ch + a.vol_off(z) + (long long)s3 * PLANE * a.es;
-            mix_lines<false, BIG>(ColLoadReal{in, n1, n2, a.es}, ColStoreHalf{S, P1, nk1, n1, n2}, g.a1, npairs, g.lg, 0,
-                                  tile, g.tsz);
-        } else if constexpr (KIND == 1) {
-            float* out = a.vol + ch + a.vol_off(z) + (long long)s3 * PLANE * a.es;
-            mix_lines<true, BIG>(ColLoadPair{S, P1, nk1, n1, n2}, ColStoreReal{out, n1, n2, a.es, a.scale}, g.a1, npairs,
-                                 g.lg, 0, tile, g.tsz);
+            const int es = KIND == kMixUnshrink ? 1 : a.es;
+            if constexpr (KIND == kMixUnshrink) in = reinterpret_cast<const float*>(slab);
+            mix_lines<false, BIG>(ColLoadReal{in, n1, n2, es}, ColStoreHalf{S, P1, nk1, n1, n2}, g.a1, npairs, g.lg, 0, tile,
+                                  g.tsz);
+            mix_lines<false, BIG>(RowLoadS{S, P1}, RowStoreBox{slab, P1, b2, k2hi}, g.a2, nk1, lgr, 1, tile, g.tsz);
         } else {
-            const float tau = a.tau[it.s - 1];
-            float2* vals = tile + 2 * g.tsz + (BIG ? n1 : 0);
-            for (int l0 = 0; l0 < npairs; l0 += 1 << g.lg) {
-                const MixTile t{l0, npairs, g.lg, 0};
-                mix_pass<true, BIG>(ColLoadPair{S, P1, nk1, n1, n2}, ColStoreShrink{vals, g.a1.pitch, l0, a.scale, tau},
-                                    g.a1, t, tile, tile + g.tsz, tile + 2 * g.tsz, 0);
-                __syncthreads();
-                mix_pass<false, BIG>(ColLoadTile{vals, g.a1.pitch, l0}, ColStoreHalf{S, P1, nk1, n1, n2}, g.a1, t, tile,
-                                     tile + g.tsz, tile + 2 * g.tsz, 0);
-                __syncthreads();
+            mix_lines<true, BIG>(RowLoadBox{slab, P1, b2, k2hi}, RowStoreS{S, P1}, g.a2, nk1, lgr, 1, tile, g.tsz);
+            const ColLoadPair ld{S, P1, nk1, n1, n2};
+            if constexpr (KIND == kMixInv) {
+                float* out = a.vol + ch + a.vol_off(z) + (long long)s3 * PLANE * a.es;
+                mix_lines<true, BIG>(ld, ColStoreReal{out, n1, n2, a.es, a.scale}, g.a1, npairs, g.lg, 0, tile, g.tsz);
+            } else {
+                mix_lines<true, BIG>(ld, ColStoreShrink{reinterpret_cast<float*>(slab), n1, n2, a.scale, a.tau[it.s - 1]},
+                                     g.a1, npairs, g.lg, 0, tile, g.tsz);
             }
         }
-        if constexpr (KIND != 1)
-            mix_lines<false, BIG>(RowLoadS{S, P1}, RowStoreBox{slab, P1, b2, k2hi}, g.a2, nk1, lgr, 1, tile, g.tsz);
     }
 }
 
-size_t mix_slab_smem(const MixSlabGeom& g, int P1, int kind) {
-    const size_t tiles = (kind != 1 || g.big ? 2 : 1) + (kind == 2 ? 1 : 0);
-    return sizeof(float2) * ((size_t)P1 * g.n2 + tiles * g.tsz + (g.big ? std::max(g.n1, g.n2) : 0));
+// Tiles of a pass: a forward one stages whole lines in a second tile.
+int mix_slab_tiles(const MixSlabGeom& g, bool fwd) { return fwd || g.big ? 2 : 1; }
+
+size_t mix_slab_smem(const MixSlabGeom& g, int P1, int tiles) {
+    return sizeof(float2) * ((size_t)P1 * g.n2 + (size_t)tiles * g.tsz + (g.big ? std::max(g.n1, g.n2) : 0));
 }
 
-// Tiles of 32 lines where two CTAs then share an SM, else of fewer.
-bool mix_slab_geom(const MixArgs& a1, const MixArgs& a2, int P1, int kind, MixSlabGeom& g) {
+// Tiles of 32 or 16 lines where two CTAs then share an SM, else of as many as
+// one CTA holds (two CTAs of 8 lines each were the slower: 160 x 124 x 96
+// analysis 764 us, one CTA of 32 lines 493).
+bool mix_slab_geom(const MixArgs& a1, const MixArgs& a2, int P1, bool fwd, MixSlabGeom& g, int more = 0) {
     g.a1 = a1;
     g.a2 = a2;
     g.n1 = a1.sc.n;
     g.n2 = a2.sc.n;
     g.big = mix_big(a1.sc) || mix_big(a2.sc);
     const int pitch = std::max(a1.pitch, a2.pitch);
-    for (size_t limit : {kMixSlabTwo, kSlabSmemOneCta})
-        for (g.lg = 5; g.lg >= 3; --g.lg) {
+    for (const bool two : {true, false})
+        for (g.lg = 5; g.lg >= (two ? 4 : 3); --g.lg) {
             g.tsz = pitch << g.lg;
-            if (mix_slab_smem(g, P1, kind) <= limit) return true;
+            if (mix_slab_smem(g, P1, mix_slab_tiles(g, fwd) + more) <= (two ? kMixSlabTwo : kSlabSmemOneCta)) return true;
         }
     return false;
 }
@@ -270,7 +271,7 @@ void launch_mix_slab_b(const SlabArgs& a, const MixSlabGeom& g, int sms, cudaStr
     auto kern = ns_mix_slab_kernel<KIND, BIG>;
     static DeviceOnce once;
     allow_smem(once, kern, kSlabSmemOneCta);
-    const size_t smem = mix_slab_smem(g, a.P1, KIND);
+    const size_t smem = mix_slab_smem(g, a.P1, mix_slab_tiles(g, KIND == kMixFwd || KIND == kMixUnshrink));
     const int items = std::max(mix_items(g.a1.sc), mix_items(g.a2.sc)) << g.lg;
     const int threads = std::min(kMixSlabThreads, std::max(64, (items + 31) / 32 * 32));
     // the last geometry's answer: the query costs as much as a launch
@@ -292,7 +293,8 @@ void launch_mix_slab_b(const SlabArgs& a, const MixSlabGeom& g, int sms, cudaStr
 template <int KIND>
 void launch_mix_slab_kind(const NSPlan& P, const SlabArgs& a, cudaStream_t st, const char* tag) {
     MixSlabGeom g;
-    if (!mix_slab_geom(mix_args(*P.ffts.at(P.dims[0])), mix_args(*P.ffts.at(P.dims[1])), P.P1, KIND, g))
+    if (!mix_slab_geom(mix_args(*P.ffts.at(P.dims[0])), mix_args(*P.ffts.at(P.dims[1])), P.P1,
+                       KIND == kMixFwd || KIND == kMixUnshrink, g))
         throw ArgError("no slab kernel for this size");
     if (g.big)
         launch_mix_slab_b<KIND, true>(a, g, P.sms, st, tag);

@@ -60,3 +60,19 @@ def test_masked_lines_of_two_radices(sfl, n3):
     ws.set_pipeline("lines")
     ref = N.analyze(N.make_tables(N.NSParams.make(**kw), dims), x)
     assert np.linalg.norm(sfl.to_host(sfl.analyze(ws, sfl.to_device(x))) - ref) <= 1e-5 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("dims,levels", [((64, 200, 20), [1, 2]), ((34, 18, 12), [1]), ((17, 13, 19), [1]), ((109, 34, 16), [2]),
+                                         ((20, 111, 18), [1, 2]), ((200, 96, 16), [1, 3]), ((12, 14, 10), [1])])
+def test_denoiser_of_run_time_slabs(sfl, dims, levels):
+    """Slabs of run-time radices threshold into the spectrum's own block between
+    two passes: bit for bit the three calls, odd counts of columns among them."""
+    ws = sfl.make_workspace(sfl.NSSurfacelet(direction_levels=levels, bernstein_order=4), "float32", dims)
+    assert ws.tuning()[0] == "mixed"
+    x = sfl.to_device(np.random.default_rng(10).standard_normal(dims).astype(np.float32))
+    c = sfl.analyze(ws, x)
+    s = torch.sign(c) * (c.abs() - 0.1).clamp(min=0)
+    s[..., 0] = c[..., 0]
+    y = sfl.denoise(ws, x, 0.1)
+    assert torch.equal(y, sfl.synthesize(ws, sfl.as_colmajor(s)))
+    assert torch.equal(y, sfl.denoise(ws, x, 0.1))
