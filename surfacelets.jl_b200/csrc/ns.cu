@@ -851,12 +851,15 @@ void ns_stream_synth_push(NSPlan& P, const void* band, cudaStream_t st) {
     {
         const long long E = ns_spec_elems(P);
         if (P.stream_pos == 0) {
-            for (int ch = 0; ch < P.nch; ++ch) ns_acc_clear(P, P.acc.as<float2>() + ch * E, ns_comp_grid(P, ch), st);
+            if (P.slab)
+                ns_slab_clear(P, st);
+            else
+                for (int ch = 0; ch < P.nch; ++ch) ns_acc_clear(P, P.acc.as<float2>() + ch * E, ns_comp_grid(P, ch), st);
             P.stream_chunk0 = 0;
         }
         if (P.slab || P.nch == 1) {
-            // stage the subband in the work slot of its position in the mask
-            // group; the axis-3 accumulation runs once per group
+            // stage the subband in the work slot of its position in the launch
+            // chunk; the axis-3 accumulation runs once per chunk
             const int c0 = P.stream_chunk0, c1 = ns_next_chunk(P, c0);
             ns_stage_range(P, reinterpret_cast<const float*>(band), ZMap{}, P.nch, P.stream_pos, 1,
                            P.stream_pos - c0, P.nch, st);

@@ -105,6 +105,28 @@ struct L3LoadSum {
     __device__ __forceinline__ float2 get(const Ctx& c, int i) const { return gs.at(c.o + i * s3); }
 };
 
+// The accumulators summed into the first one, two bins a thread and step (the
+// pitch is even and every accumulator starts 16-byte aligned).
+template <int NG>
+__global__ void __launch_bounds__(256) sum_groups_kernel(float4* acc, const float4* comp, long long gstride, long long n) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        float4 s[NG], e[NG];
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+            s[g] = acc[g * gstride + i];
+            e[g] = __ldg(comp + g * gstride + i);
+        }
+        float2 a = c_sub(make_float2(s[0].x, s[0].y), make_float2(e[0].x, e[0].y));
+        float2 b = c_sub(make_float2(s[0].z, s[0].w), make_float2(e[0].z, e[0].w));
+#pragma unroll
+        for (int g = 1; g < NG; ++g) {
+            a = c_add(a, c_sub(make_float2(s[g].x, s[g].y), make_float2(e[g].x, e[g].y)));
+            b = c_add(b, c_sub(make_float2(s[g].z, s[g].w), make_float2(e[g].z, e[g].w)));
+        }
+        acc[i] = make_float4(a.x, a.y, b.x, b.y);
+    }
+}
+
 // A channel's accumulators added into a caller's spectrum and its compensation
 // (on a cleared one, GroupSum's values exactly).
 template <int NG>
@@ -408,6 +430,20 @@ void slab_rfft3(NSPlan& P, const float* x, int es, float2* X, int nch, cudaStrea
                  "ns_slab_line3");
 }
 
+void sum_groups(NSPlan& P, float2* A, const float2* K, int ng, int nch, cudaStream_t st) {
+    const long long n = nch * P.SP / 2, blocks = std::min<long long>((n + 255) / 256, 16LL * P.sms);
+    float4* a = reinterpret_cast<float4*>(A);
+    const float4* k = reinterpret_cast<const float4*>(K);
+    const long long gs = (long long)P.nch * P.SP / 2;
+    int tok = prof_begin("ns_slab_line3", st);
+    if (ng == 4)
+        sum_groups_kernel<4><<<(unsigned)blocks, 256, 0, st>>>(a, k, gs, n);
+    else
+        sum_groups_kernel<2><<<(unsigned)blocks, 256, 0, st>>>(a, k, gs, n);
+    prof_end(tok, st);
+    cuda_check(cudaGetLastError(), "sum_groups_kernel launch");
+}
+
 // irfft3 of the padded spectra A + ch SP (overwritten) into nch channels.
 void slab_irfft3(NSPlan& P, float2* A, float* x, int es, int nch, cudaStream_t st) {
     const NSBox& full = P.boxes_full;
@@ -419,7 +455,13 @@ void slab_irfft3(NSPlan& P, float2* A, float* x, int es, int nch, cudaStream_t s
     const L3StoreC so{A, P.SP, P.P1, s3, bx};
     const float2* K = P.comp.as<float2>() + (ng > 1 ? A - P.acc.as<float2>() : 0);
     const long long gs = (long long)P.nch * P.SP;
-    if (ng == 4)
+    // the register pass holds 24 or 40 values a thread at 96 and 160 points, too many beside their sums' loads: the
+    // accumulators are summed ahead of it there (64 x 64 x 160: 29 -> 12 us, 96 cubed 14 -> 10; one launch more
+    // elsewhere gains nothing)
+    if (ng > 1 && (P.dims[2] == 96 || P.dims[2] == 160)) {
+        sum_groups(P, A, K, ng, nch, st);
+        line3<true>(P, L3LoadC{A, P.SP, P.P1, s3, bx}, so, nl, nch, st, "ns_slab_line3");
+    } else if (ng == 4)
         line3<true>(P, L3LoadSum<4>{{A, K, gs}, P.SP, P.P1, s3, bx}, so, nl, nch, st, "ns_slab_line3");
     else if (ng == 2)
         line3<true>(P, L3LoadSum<2>{{A, K, gs}, P.SP, P.P1, s3, bx}, so, nl, nch, st, "ns_slab_line3");
@@ -590,6 +632,12 @@ void ns_slab_acc_clear(NSPlan& P, float2* acc, float2* comp, cudaStream_t st) {
     }
 }
 
+void ns_slab_clear(NSPlan& P, cudaStream_t st) {
+    const size_t bytes = sizeof(float2) * P.SP * P.nch * P.ngrp;
+    cuda_check(cudaMemsetAsync(P.acc.p, 0, bytes, st), "cudaMemsetAsync(acc)");
+    cuda_check(cudaMemsetAsync(P.comp.p, 0, bytes, st), "cudaMemsetAsync(comp)");
+}
+
 void ns_merge_groups(NSPlan& P, int ch, float2* A, float2* C, cudaStream_t st) {
     const long long blocks = std::min<long long>((P.SP + 255) / 256, 8LL * P.sms);
     const float2 *a = P.acc.as<float2>() + ch * P.SP, *k = P.comp.as<float2>() + ch * P.SP;
@@ -647,8 +695,7 @@ void ns_slab_synthesize(NSPlan& P, const void* c, void* x, cudaStream_t st, bool
     const int nch = P.nch;
     float2* A = P.acc.as<float2>();
     float2* K = P.comp.as<float2>();
-    cuda_check(cudaMemsetAsync(A, 0, sizeof(float2) * P.SP * nch * P.ngrp, st), "cudaMemsetAsync(acc)");
-    cuda_check(cudaMemsetAsync(K, 0, sizeof(float2) * P.SP * nch * P.ngrp, st), "cudaMemsetAsync(comp)");
+    ns_slab_clear(P, st);
     for (int i0 = 0, i1; i0 < P.S; i0 = i1) {
         i1 = chunk_end(P, i0);
         slab_synth_items(P, static_cast<const float*>(c), ns_subband_map(P, i0, nch), nch, i0, i1 - i0,

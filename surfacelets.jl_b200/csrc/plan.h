@@ -217,6 +217,8 @@ bool ns_mix_slab_supported(const NSPlan& P);
 void ns_use_mixed(NSPlan& P);
 int ns_slab_groups(const NSPlan& P);
 void ns_slab_acc_clear(NSPlan& P, float2* acc, float2* comp, cudaStream_t st);
+// Clears the plan's accumulators, every channel's.
+void ns_slab_clear(NSPlan& P, cudaStream_t st);
 // The plan's accumulators of channel ch added into a caller's spectrum A with compensation C.
 void ns_merge_groups(NSPlan& P, int ch, float2* A, float2* C, cudaStream_t st);
 // Compensation of a caller's spectrum: the plan's own grid, or with several accumulators one beside theirs.

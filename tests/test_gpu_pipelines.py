@@ -76,3 +76,24 @@ def test_denoiser_of_run_time_slabs(sfl, dims, levels):
     y = sfl.denoise(ws, x, 0.1)
     assert torch.equal(y, sfl.synthesize(ws, sfl.as_colmajor(s)))
     assert torch.equal(y, sfl.denoise(ws, x, 0.1))
+
+
+@pytest.mark.parametrize("dims,dtype", [((64, 64, 160), "float32"), ((64, 64, 96), "complex64"), ((96, 96, 96), "complex64"),
+                                        ((30, 20, 96), "float32"), ((128, 64, 160), "float32")])
+def test_accumulators_summed_ahead_of_the_inverse(sfl, dims, dtype):
+    """Two and four accumulators with 96 and 160 points along axis 3: against the
+    line pipeline's one (a few float32 roundings apart, bar 1e-6), and streamed
+    bit for bit."""
+    rng = np.random.default_rng(11)
+    t = sfl.NSSurfacelet(direction_levels=[1, 2], bernstein_order=6)
+    ws, wl = sfl.make_workspace(t, dtype, dims), sfl.make_workspace(t, dtype, dims)
+    wl.set_pipeline("lines")
+    c = rng.standard_normal(dims + (ws.nsubbands,)).astype(np.float32)
+    if dtype == "complex64":
+        c = (c + 1j * rng.standard_normal(c.shape)).astype(np.complex64)
+    c = sfl.to_device(c)
+    y, z = sfl.synthesize(ws, c), sfl.synthesize(wl, c)
+    assert float(torch.linalg.vector_norm(y - z) / torch.linalg.vector_norm(z)) <= 1e-6
+    s = sfl.volume_like(dims, dtype)
+    sfl.synthesize_(lambda i: c[..., i - 1], s, ws)
+    assert torch.equal(s, y)
