@@ -328,22 +328,25 @@ __device__ __forceinline__ void irc_plane_seg_fft(int ap, int a1, int a2, bool a
 }
 
 // A function of its own per length: inlined, the 82 lengths would make one
-// kernel too large to compile.  The powers of two are inlined: as calls, under
-// the 64 registers of a 1024-thread CTA, the 128^3 planes took 73 and 64 us
-// (analysis, synthesis) instead of 63 and 57.
+// kernel too large to compile.  The powers of two are inlined, in a kernel
+// without the calls (POW2): under the 64 registers of a 1024-thread CTA the
+// synthesis planes of 128^3 take 58 us there, 61 with the calls beside them and
+// 64 as calls (analysis 72, 72 and 73).
 template <int N, bool INV>
 __device__ __noinline__ void irc_plane_seg_fft_call(int ap, int a1, int a2, bool along1, int to) {
     irc_plane_seg_fft<N, INV>(ap, a1, a2, along1, to);
 }
 
-template <bool INV>
+__host__ inline bool irc_plane_pow2(int n) { return (n & (n - 1)) == 0; }   // 0 (run separately) among them
+
+template <bool INV, bool POW2>
 __device__ __forceinline__ void irc_plane_block_ffts(int ap, int a1, int a2, int bs, bool along1, int to) {
     switch (bs) {
 #define SFL_ANY_CASE(N_)                                                     \
     case N_:                                                                 \
         if constexpr ((N_ & (N_ - 1)) == 0)                                  \
             irc_plane_seg_fft<N_, INV>(ap, a1, a2, along1, to);              \
-        else                                                                 \
+        else if constexpr (!POW2)                                            \
             irc_plane_seg_fft_call<N_, INV>(ap, a1, a2, along1, to);         \
         break;
         SFL_ANY_LENGTHS(SFL_ANY_CASE)
@@ -360,7 +363,7 @@ __device__ __forceinline__ void irc_plane_load_twiddles(float2* tw2s, const floa
     }
 }
 
-template <bool SYNTH>
+template <bool SYNTH, bool POW2>
 __global__ void __launch_bounds__(kIrcPlaneThreads) irc_plane_kernel(const __grid_constant__ IrcPlaneJobs jobs) {
     float2* const pl = irc_sm;
     int t0 = 0;
@@ -431,9 +434,9 @@ __global__ void __launch_bounds__(kIrcPlaneThreads) irc_plane_kernel(const __gri
     __syncthreads();
     if (SYNTH && fused) {
         // subband -> block: the forward block FFTs along both transverse axes, then the stages in reverse
-        irc_plane_block_ffts<false>(ap, a1, a2, jb.bs1, true, (int)(tws - pl));
+        irc_plane_block_ffts<false, POW2>(ap, a1, a2, jb.bs1, true, (int)(tws - pl));
         __syncthreads();
-        irc_plane_block_ffts<false>(ap, a1, a2, jb.bs2, false, (int)(tws - pl) + jb.bs1);
+        irc_plane_block_ffts<false, POW2>(ap, a1, a2, jb.bs2, false, (int)(tws - pl) + jb.bs1);
         __syncthreads();
     }
     for (int t = 0; t < sg.n; ++t) {
@@ -481,9 +484,9 @@ __global__ void __launch_bounds__(kIrcPlaneThreads) irc_plane_kernel(const __gri
     }
     if (!SYNTH && fused) {
         // block -> subband, first half: the inverse block FFTs along both transverse axes
-        irc_plane_block_ffts<true>(ap, a1, a2, jb.bs1, true, (int)(tws - pl));
+        irc_plane_block_ffts<true, POW2>(ap, a1, a2, jb.bs1, true, (int)(tws - pl));
         __syncthreads();
-        irc_plane_block_ffts<true>(ap, a1, a2, jb.bs2, false, (int)(tws - pl) + jb.bs1);
+        irc_plane_block_ffts<true, POW2>(ap, a1, a2, jb.bs2, false, (int)(tws - pl) + jb.bs1);
         __syncthreads();
     }
     for (int q = threadIdx.x; q < tot; q += blockDim.x) {
@@ -1063,12 +1066,6 @@ IrcPlaneStages irc_plane_stages(const DecLevelDev& L, int K, bool synth) {
     return ps;
 }
 
-template <bool SYNTH>
-void irc_plane_configure() {
-    static DeviceOnce once;
-    allow_smem(once, irc_plane_kernel<SYNTH>, 227 * 1024);
-}
-
 // Whether the plane pass of level L runs hourglass K (its plane fits; the
 // synthesis has nothing to do without stages) and whether it runs K's block
 // FFTs too.
@@ -1090,16 +1087,20 @@ void irc_plane_launch_levels(DecPlan& D, cudaStream_t st, bool adjoint = false) 
     IrcPlaneJobs jobs{};
     size_t smem = 0;
     int blocks = 0;
+    bool pow2 = true;
     auto flush = [&] {
         if (jobs.n == 0) return;
-        irc_plane_configure<SYNTH>();
+        auto kern = pow2 ? irc_plane_kernel<SYNTH, true> : irc_plane_kernel<SYNTH, false>;
+        static DeviceOnce once[2];
+        allow_smem(once[pow2], kern, 227 * 1024);
         int tok = prof_begin("dec_irc_plane", st);
-        irc_plane_kernel<SYNTH><<<blocks, kIrcPlaneThreads, smem, st>>>(jobs);
+        kern<<<blocks, kIrcPlaneThreads, smem, st>>>(jobs);
         prof_end(tok, st);
         cuda_check(cudaGetLastError(), "irc_plane_kernel");
         jobs = IrcPlaneJobs{};
         smem = 0;
         blocks = 0;
+        pow2 = true;
     };
     for (int j = 0; j < D.J; ++j) {
         DecLevelDev& L = *D.lv[j];
@@ -1128,6 +1129,7 @@ void irc_plane_launch_levels(DecPlan& D, cudaStream_t st, bool adjoint = false) 
                 jb.bs2 = L.bsize[K][m2];
                 jb.tw1 = get_fft(D.ffts, jb.bs1)->sh.tw;
                 jb.tw2 = get_fft(D.ffts, jb.bs2)->sh.tw;
+                pow2 = pow2 && irc_plane_pow2(jb.bs1) && irc_plane_pow2(jb.bs2);
             }
             blocks += L.hd[K][K];
             smem = std::max(smem, irc_plane_smem(L, K));
