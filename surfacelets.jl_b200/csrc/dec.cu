@@ -840,17 +840,6 @@ Lines block_lines(const int hd[3], int m, int bl) {
     return g;
 }
 
-// Segmented FFTs along axis m of a half-K spectrum: blocks of length bl.
-void block_fft(DecPlan& D, float2* S, const int hd[3], int m, int bl, bool inv, cudaStream_t st) {
-    const Lines g = block_lines(hd, m, bl);
-    FFTLen* f = get_fft(D.ffts, bl);
-    const bool tf = g.si != 1;
-    if (inv)
-        launch_line<true>(*f, RLoadC{S, ZMap{}, g}, RStoreC{S, ZMap{}, g}, g.nlines, 1, tf, st, "dec_block_fft");
-    else
-        launch_line<false>(*f, RLoadC{S, ZMap{}, g}, RStoreC{S, ZMap{}, g}, g.nlines, 1, tf, st, "dec_block_fft");
-}
-
 // Block FFTs of several spectra in one pass: item z (grid.y) has its
 // own spectrum and line geometry (same length); lines past an item's count
 // read zeros and store nothing.
@@ -1078,10 +1067,10 @@ bool irc_plane_fuses(const DecLevelDev& L, int K) {
     return irc_plane_runs<SYNTH>(L, K) && irc_plane_fuses_blocks(L, K);
 }
 
-// One launch of the plane pass over every level's hourglasses whose plane
-// fits, or its transpose (analysis: with the mask on load from the level spectrum; synthesis:
-// hourglasses without stages have nothing to do), the finest level's planes
-// first so that the coarser levels' smaller planes fill the last wave.
+// One launch of the plane pass, or its transpose, over every level's hourglasses
+// whose plane fits (analysis: with the mask on load from the level spectrum;
+// synthesis: hourglasses without stages have nothing to do), the finest level's
+// planes first so that the coarser levels' smaller planes fill the last wave.
 template <bool SYNTH>
 void irc_plane_launch_levels(DecPlan& D, cudaStream_t st, bool adjoint = false) {
     IrcPlaneJobs jobs{};

@@ -17,8 +17,9 @@
 //     slab pass  per n3: R2C along axis 1 (two columns at a time), FFT_2 of
 //                the rows in the box -> Y_s;
 //     line pass  FFT_3 of Y_s times M_s, summed over the subbands of one mask
-//                group in registers, then one Kahan-compensated step into the
-//                accumulator (a round trip of it and its compensation per group);
+//                group on chip (with a Kahan step a term on mixed plans), then
+//                one Kahan step into the accumulator (a round trip of it and its
+//                compensation per group);
 //     then the irfft of the accumulator (line pass and slab pass, no mask).
 //
 // Support boxes: the group factor B_j of scale j is a product of per-axis
